@@ -60,6 +60,15 @@ __device__ __forceinline__ float block_max(float v, float* red) {
   return r;
 }
 
+// Programmatic dependent launch: a kernel launched with the attribute may start once every CTA of the kernel before
+// it has called let_next_kernel_start (or left), and sees that kernel's results after wait_for_previous_kernel.
+// Both do nothing in an ordinary launch.  Data of the kernel before must not be read through const __restrict__
+// pointers: the compiler may move such loads in front of the wait.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 // 16-byte vector of 8 bf16 values.
 struct __align__(16) bf16x8 {
   __nv_bfloat162 v[4];
@@ -78,6 +87,38 @@ __device__ __forceinline__ bf16x8 pack8(const float* f) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) p.v[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
   return p;
+}
+
+// Two fp32 values in one 64-bit register: sm_100 issues one instruction for both (element 0 in the low half).
+typedef uint64_t f32x2;
+__device__ __forceinline__ f32x2 pack_f32x2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add_f32x2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// bf16 pair -> fp32 pair (a bf16 is the upper half of an fp32)
+__device__ __forceinline__ f32x2 bf16x2_to_f32x2(uint32_t p) {
+  return pack_f32x2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
 }
 
 // tanh on the special-function unit (max abs error ~5e-4, far below bf16 resolution).

@@ -418,24 +418,25 @@ class ParallelMHA(nn.Module):
         b, s = qkv.shape[:2]
         hq, hk, d = self.local_heads, self.local_heads_kv, self.head_dim
         off = ip.seqlen_offset
-        if hq == hk:
-            qkv = qkv.view(b, s, 3, hq, d)
-            if self.rotary_emb_dim > 0:
-                cos, sin = F.rope_tables(ip.max_seqlen, self.rotary_emb_dim, self.rotary_emb_base, qkv.device)
-                qkv = F.apply_rotary_qkv_(qkv.contiguous(), cos[off:off + s], sin[off:off + s], self.rotary_emb_dim)
-            q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
+        rotary = None
+        if self.rotary_emb_dim > 0:
+            cos, sin = F.rope_tables(ip.max_seqlen, self.rotary_emb_dim, self.rotary_emb_base, qkv.device)
+            rotary = (cos[off:off + s], sin[off:off + s], self.rotary_emb_dim)
+        cache = ip.cache_for(self.layer_idx, b, hk, d, qkv.dtype, qkv.device)      # [b, max_seq, 2, hk, d]
+        if F.rope_append_available(qkv, cache, self.rotary_emb_dim, d):
+            assert off + s <= cache.shape[1], "sequence longer than the cache was sized for"
+            F.rope_append_(qkv, cache, off, hq, hk, d, rotary)
+            q = qkv[..., : hq * d].view(b, s, hq, d)
+            k, v = cache[:b, off:off + s, 0], cache[:b, off:off + s, 1]
         else:
             qk = qkv[..., : (hq + hk) * d].reshape(b, s, 1, hq + hk, d)
-            if self.rotary_emb_dim > 0:
-                cos, sin = F.rope_tables(ip.max_seqlen, self.rotary_emb_dim, self.rotary_emb_base, qkv.device)
-                qk = F._rope_apply(qk.contiguous().clone(), cos[off:off + s], sin[off:off + s], self.rotary_emb_dim,
-                                   False, 1)
+            if rotary is not None:
+                qk = F._rope_apply(qk.contiguous().clone(), *rotary, False, 1)
             qk = qk.reshape(b, s, hq + hk, d)
             q, k = qk[:, :, :hq], qk[:, :, hq:]
             v = qkv[..., (hq + hk) * d:].reshape(b, s, hk, d)
-        cache = ip.cache_for(self.layer_idx, b, hk, d, qkv.dtype, qkv.device)      # [b, max_seq, 2, hk, d]
-        cache[:b, off:off + s, 0].copy_(k)
-        cache[:b, off:off + s, 1].copy_(v)
+            cache[:b, off:off + s, 0].copy_(k)
+            cache[:b, off:off + s, 1].copy_(v)
         if s == 1:
             ctx = F.decode_attention(q[:, 0], cache[:b, :, 0], cache[:b, :, 1], off + 1, self.softmax_scale)
             ctx = ctx.unsqueeze(1)

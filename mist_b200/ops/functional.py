@@ -720,12 +720,30 @@ def decode_attention(q, k_cache, v_cache, seq_len: int, scale: Optional[float] =
             v = v.repeat_interleave(nh // nkv, dim=2)
         s = torch.einsum("bhd,bkhd->bhk", q.float(), k) * scale
         return torch.einsum("bhk,bkhd->bhd", torch.softmax(s, dim=-1), v).to(q.dtype)
-    q = q.contiguous()
-    out = torch.empty_like(q)
+    if q.stride(2) != 1 or q.stride(1) != d or q.stride(0) % 8:
+        q = q.contiguous()
+    out = torch.empty(b, nh, d, dtype=q.dtype, device=q.device)
     ks, vs = k_cache.stride(), v_cache.stride()
     call("mb_decode_attn", ptr(q), ptr(k_cache), ptr(v_cache), ptr(out), b, nh, nkv, d, int(seq_len),
-         ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], scale, stream())
+         q.stride(0), ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], scale, 0, stream())
     return out
+
+
+def rope_append_available(qkv, cache, rot: int, d: int) -> bool:
+    return (not _sym(qkv) and use_native(qkv) and qkv.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16
+            and d % 8 == 0 and rot % 16 == 0)
+
+
+def rope_append_(qkv, cache, offset: int, hq: int, hk: int, d: int, rotary=None):
+    """New tokens of cached generation: rotates q of the packed projection output ``[b, s, (hq + 2 hk) d]`` in place
+    and writes the rotated k and v to rows ``offset ...`` of ``cache`` ``[>= b, max_seq, 2, hk, d]``, one kernel.
+    ``rotary``: ``None`` or ``(cos, sin, rot_dim)`` whose first row belongs to position ``offset``.  k inside ``qkv``
+    keeps its unrotated values."""
+    b, s = qkv.shape[:2]
+    assert qkv.is_contiguous() and cache.stride()[1:] == (2 * hk * d, hk * d, d, 1)
+    cos, sin, rot = rotary if rotary is not None else (None, None, 0)
+    call("mb_rope_append", ptr(qkv), ptr(cache), ptr(cos), ptr(sin), b, s, hq, hk, d, int(rot), int(offset),
+         cache.stride(0), 0, stream())
 
 
 def _ref_attention(q, k, v, scale, causal, seqlens_q=None, seqlens_k=None):
