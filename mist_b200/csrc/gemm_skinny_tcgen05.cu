@@ -1,0 +1,350 @@
+// bf16 linear layer for a handful of tokens (decoding, short prompts):
+//
+//   y[M, N] = epi(x[M, K] W[N, K]^T),  M <= 128        epi: + bias, GELU, + residual, or SwiGLU over [gate | up]
+//
+// Bound: reading W once from HBM.  The ordinary GEMM tiles put the tokens on the 128-row side of the MMA and give a
+// CTA 128 columns of W, so a 4096 x 4096 layer ran on 32 CTAs of 148 (39 us for 33.6 MB, 0.9 TB/s).  Here
+//   * W is the 128-row operand and the tokens are the 16 .. 128 columns, so no MMA row is padding;
+//   * the CTAs of a cluster (up to eight) share the K range of a tile and sum their fp32 partial tiles through
+//     distributed shared memory in rank order: enough CTAs for any N, one launch, no workspace, the same bits on
+//     every run;
+//   * four 18 - 24 KB stages and two or three CTAs per SM keep about 200 KB of W per SM in flight;
+//   * W does not depend on the kernel before: launched as a programmatic dependent (`pdl`), the CTAs start to load W
+//     while that kernel drains and wait for it only before they read x.  The caller may ask for that only where no
+//     kernel still running can write W.
+// Warps: 0 TMA, 1 MMA, 2 - 5 read the accumulator; all six finish the outputs.
+//
+// Reference counterpart: the cuBLAS calls of csrc/fused_dense_lib/fused_dense_cuda.cu:19-92 at small batch.
+#include "sm100_pair.cuh"
+#include <string.h>
+
+using namespace sm100;
+
+namespace {
+
+constexpr int BR = 128;       // rows of W per CTA (64 gate + 64 up rows in the SwiGLU form)
+constexpr int BK = 64;
+constexpr int kThreads = 192;
+constexpr int kStages = 4;
+constexpr int kMaxSplit = 8;
+
+enum EpiFlags : int { EPI_BIAS = 1, EPI_GELU = 2, EPI_RESIDUAL = 64, EPI_SWIGLU = 128 };
+
+struct SkinnyParams {
+  int M, N, K;               // N: output columns
+  __nv_bfloat16* C;
+  int ldc;
+  const __nv_bfloat16* bias;
+  const __nv_bfloat16* aux;  // residual, [M][N] with row stride ldc
+  int flags;
+  float alpha;
+  int* status;
+};
+
+template <int NT>
+struct SkinnyLayout {
+  static constexpr int kW = BR * BK * 2;
+  static constexpr int kX = NT * BK * 2;
+  static constexpr int kStage = kW + kX;
+  static constexpr int kPartStride = BR + 4;                      // floats per token of the partial tile
+  static constexpr int kPart = NT * kPartStride * 4;              // over the stages, once they have been read
+  static constexpr int kRing = kStages * kStage;
+  static constexpr int kBarOffset = kRing > kPart ? kRing : kPart;
+  static constexpr int kTotal = kBarOffset + (2 * kStages + 1) * 8 + 16;
+};
+
+__device__ __forceinline__ void report(int* status, int code) {
+  if (status) atomicCAS(status, 0, code);
+}
+__device__ __forceinline__ float2 ld_cluster2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kThreads)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x,
+                   const SkinnyParams p) {
+  using L = SkinnyLayout<NT>;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kBarOffset);
+  uint64_t* empty_bar = full_bar + kStages;
+  uint64_t* done_bar = empty_bar + kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = gridDim.x, rank = blockIdx.x;
+  const bool swiglu = (p.flags & EPI_SWIGLU) != 0;
+  const int width = swiglu ? BR / 2 : BR;            // output columns of this tile
+  const int n0 = blockIdx.y * width;
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int kb0 = static_cast<int>(static_cast<long>(num_kb) * rank / split);
+  const int kb1 = static_cast<int>(static_cast<long>(num_kb) * (rank + 1) / split);
+  constexpr int kTmemCols = NT < 32 ? 32 : NT;
+
+  mb::let_next_kernel_start();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(done_bar, 1);
+    fence_barrier_init();
+    prefetch_tmap(&tma_w);
+    prefetch_tmap(&tma_x);
+  }
+  if (warp == 2) {
+    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      uint32_t armed[kStages];
+      for (int s = 0; s < kStages; ++s) armed[s] = 0;
+      const int row_a = n0, row_b = swiglu ? p.N + n0 : n0 + BR / 2;
+      auto load_w = [&](int i) {
+        const int s = i % kStages;
+        uint8_t* sw = smem + s * L::kStage;
+        mbar_expect_tx(&full_bar[s], L::kStage);
+        armed[s]++;
+        tma_load_2d(sw, &tma_w, &full_bar[s], (kb0 + i) * BK, row_a);
+        tma_load_2d(sw + L::kW / 2, &tma_w, &full_bar[s], (kb0 + i) * BK, row_b);
+      };
+      auto load_x = [&](int i) {
+        const int s = i % kStages;
+        tma_load_2d(smem + s * L::kStage + L::kW, &tma_x, &full_bar[s], (kb0 + i) * BK, 0);
+      };
+      const int n = kb1 - kb0, head = n < kStages ? n : kStages;
+      for (int i = 0; i < head; ++i) load_w(i);
+      mb::wait_for_previous_kernel();
+      for (int i = 0; i < head; ++i) load_x(i);
+      for (int i = head; i < n; ++i) {
+        if (!mbar_wait(&empty_bar[i % kStages], ((i / kStages) - 1) & 1)) {
+          report(p.status, MB_ERR_TIMEOUT_EMPTY);
+          ok = false;
+          break;
+        }
+        load_w(i);
+        load_x(i);
+      }
+      if (!ok) {      // gave up: let the copies already in flight land before the CTA exits
+        for (int s = 0; s < kStages; ++s)
+          if (armed[s]) mbar_wait(&full_bar[s], (armed[s] - 1) & 1, 50);
+      }
+    }
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = make_idesc_bf16(BR, NT, 0, 0);
+    bool ok = true;
+    for (int i = 0; i < kb1 - kb0; ++i) {
+      const int s = i % kStages;
+      if (!mbar_wait(&full_bar[s], (i / kStages) & 1)) {
+        report(p.status, MB_ERR_TIMEOUT_FULL);
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      if (lane == 0) {
+        const uint32_t sw = smem_u32(smem + s * L::kStage), sx = sw + L::kW;
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          mma_f16_ss(tmem_base, make_smem_desc_sw128(sw + k * 32, 16, 1024), make_smem_desc_sw128(sx + k * 32, 16, 1024),
+                     idesc, (i | k) != 0 ? 1u : 0u);
+        mma_commit(&empty_bar[s]);
+      }
+      __syncwarp();
+    }
+    if (ok && lane == 0) mma_commit(done_bar);
+    __syncwarp();
+  } else {
+    const int q = warp & 3, r = q * 32 + lane;       // accumulator lane = row of W
+    float* part = reinterpret_cast<float*>(smem);
+    if (mbar_wait(done_bar, 0)) {                    // every MMA has read its stage: the ring is free
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < NT / 16; ++c) {
+        uint32_t a[16];
+        tmem_ld16(tmem_base + c * 16 + (static_cast<uint32_t>(q * 32) << 16), a);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) part[(c * 16 + i) * L::kPartStride + r] = __uint_as_float(a[i]);
+      }
+    } else {
+      report(p.status, MB_ERR_TIMEOUT_TMEM);
+    }
+  }
+  mb::wait_for_previous_kernel();       // this thread may read the residual and overwrite C below
+  tc_fence_before();
+  __syncthreads();
+  if (split > 1) cluster_sync_all();
+
+  // two neighbouring columns per thread; the CTAs of the cluster share the outputs
+  const int pairs = width / 2;
+  const uint32_t part_u = smem_u32(smem);
+  for (int t = rank * kThreads + threadIdx.x; t < p.M * pairs; t += split * kThreads) {
+    const int m = t / pairs, c = (t - m * pairs) * 2, n = n0 + c;
+    if (n >= p.N) continue;
+    const uint32_t off = part_u + static_cast<uint32_t>(m * L::kPartStride + c) * 4;
+    float2 v = make_float2(0.f, 0.f), u = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < kMaxSplit; ++r) {
+      if (r < split) {
+        const uint32_t at = split > 1 ? map_to_cta(off, r) : off;
+        const float2 a = ld_cluster2(at);
+        v.x += a.x;
+        v.y += a.y;
+        if (swiglu) {
+          const float2 b = ld_cluster2(at + (BR / 2) * 4);
+          u.x += b.x;
+          u.y += b.y;
+        }
+      }
+    }
+    v.x *= p.alpha;
+    v.y *= p.alpha;
+    u.x *= p.alpha;
+    u.y *= p.alpha;
+    const bool two = n + 1 < p.N;
+    if (p.flags & EPI_BIAS) {
+      v.x += __bfloat162float(p.bias[n]);
+      if (two) v.y += __bfloat162float(p.bias[n + 1]);
+      if (swiglu) {
+        u.x += __bfloat162float(p.bias[p.N + n]);
+        if (two) u.y += __bfloat162float(p.bias[p.N + n + 1]);
+      }
+    }
+    if (p.flags & EPI_GELU) {
+      v.x = mb::gelu_tanh(v.x);
+      v.y = mb::gelu_tanh(v.y);
+    }
+    if (swiglu) {
+      v.x = mb::silu(v.x) * u.x;
+      v.y = mb::silu(v.y) * u.y;
+    }
+    const long o = static_cast<long>(m) * p.ldc + n;
+    if (p.flags & EPI_RESIDUAL) {
+      v.x += __bfloat162float(p.aux[o]);
+      if (two) v.y += __bfloat162float(p.aux[o + 1]);
+    }
+    if (two && (p.ldc & 1) == 0)
+      *reinterpret_cast<__nv_bfloat162*>(p.C + o) = __floats2bfloat162_rn(v.x, v.y);
+    else {
+      p.C[o] = __float2bfloat16(v.x);
+      if (two) p.C[o + 1] = __float2bfloat16(v.y);
+    }
+  }
+  if (split > 1) cluster_sync_all();      // nobody leaves while its partial tile is being read
+  __syncthreads();
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_fn() {
+  static EncodeTiledFn fn = nullptr;
+  if (!fn) {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      return nullptr;
+    fn = reinterpret_cast<EncodeTiledFn>(ptr);
+  }
+  return fn;
+}
+bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * 2};
+  cuuint32_t box[2] = {BK, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return encode_with_context([&] {
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
+}
+
+template <int NT>
+int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int tiles, int split, int pdl,
+                  cudaStream_t stream) {
+  constexpr int smem = SkinnyLayout<NT>::kTotal + 1024;
+  auto kern = gemm_skinny_kernel<NT>;
+  static const bool configured =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+  if (!configured) return -3;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(split, tiles, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, tw, tx, p) == cudaSuccess ? 0 : -4;
+}
+
+}  // namespace
+
+MB_API int* mb_status_device_ptr();
+
+// C[M, N] = epi(alpha * A[M, K] B[N, K]^T) for M <= 128, bf16 in and out.  flags: bias, GELU, residual (aux, row
+// stride ldc), or 128: SwiGLU, where B holds 2 N rows [gate | up] (and the bias 2 N values).  A and B 16-byte
+// aligned, lda and ldb multiples of 8.  Returns 1 without launching when the arguments need another kernel.
+MB_API int mb_gemm_skinny_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                               int flags, const void* bias, const void* aux, float alpha, int pdl,
+                               cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
+    return -1;
+  if (M > 128 || (flags & ~(EPI_BIAS | EPI_GELU | EPI_RESIDUAL | EPI_SWIGLU)) || (reinterpret_cast<uintptr_t>(C) & 3))
+    return 1;
+  const bool swiglu = (flags & EPI_SWIGLU) != 0;
+  if ((swiglu && (flags & EPI_GELU)) || ((flags & EPI_RESIDUAL) && !aux)) return 1;
+  if (swiglu && N % (BR / 2)) return 1;      // a tile would mix gate rows with up rows
+  const int width = swiglu ? BR / 2 : BR;
+  const int tiles = (N + width - 1) / width;
+  if (tiles > 65535) return 1;
+  const int num_kb = (K + BK - 1) / BK;
+  const int nt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  // CTAs that share a tile's K range: doubled while the grid has fewer than two CTAs per SM and a CTA keeps at
+  // least four k-blocks (one ring).
+  int split = 1;
+  while (split < kMaxSplit && static_cast<long>(tiles) * split < 2L * 148 && num_kb >= 8 * split) split *= 2;
+  CUtensorMap tw, tx;
+  if (!make_map(&tw, B, static_cast<uint64_t>(N) * (swiglu ? 2 : 1), K, ldb, BR / 2)) return -2;
+  if (!make_map(&tx, A, M, K, lda, nt)) return -2;
+  SkinnyParams p;
+  p.M = M; p.N = N; p.K = K;
+  p.C = reinterpret_cast<__nv_bfloat16*>(C);
+  p.ldc = ldc;
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  p.aux = reinterpret_cast<const __nv_bfloat16*>(aux);
+  p.flags = flags;
+  p.alpha = alpha;
+  p.status = mb_status_device_ptr();
+  if (nt == 16) return launch_skinny<16>(tw, tx, p, tiles, split, pdl, stream);
+  if (nt == 32) return launch_skinny<32>(tw, tx, p, tiles, split, pdl, stream);
+  if (nt == 64) return launch_skinny<64>(tw, tx, p, tiles, split, pdl, stream);
+  return launch_skinny<128>(tw, tx, p, tiles, split, pdl, stream);
+}

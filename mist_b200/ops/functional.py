@@ -106,6 +106,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         flags |= EPI_OUT_FP32
     if bias is not None:
         flags |= EPI_BIAS
+    if M <= 128 and tile_n == 0 and not a_mn and not b_mn and out.dtype == torch.bfloat16:
+        # a few tokens: the kernel that puts W on the 128-row side and splits K (1: epilogue not covered)
+        rc = native.kernels().mb_gemm_skinny_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
+                                                  out.stride(0), flags, ptr(bias), ptr(aux), float(alpha), 0, stream())
+        if rc == 0:
+            native.launch_count += 1
+            return out
+        if rc != 1:
+            raise RuntimeError(f"mb_gemm_skinny_bf16 failed with code {rc}")
     if Settings.gemm_pair and tile_n == 0:
         # returns 1 (nothing launched) when the shape or epilogue needs the single-CTA kernel
         rc = native.kernels().mb_gemm_pair_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),

@@ -49,3 +49,21 @@ def test_rope_append(hq, hk, d, rot, s):
     keep = torch.ones(rows, dtype=torch.bool)
     keep[off:off + s] = False
     assert (cache[:b, keep.to(DEV)] == 7).all() and (cache[b] == 7).all()
+
+
+# M: the sides of every token-tile size (16, 32, 64, 128); N: one tile, a tail of one column pair and of an odd
+# column; K: one k-block, a K tail, and enough for two, four and eight CTAs per tile
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize("N,K", [(128, 64), (130, 72), (333, 1024), (384, 2056), (256, 4096)])
+def test_skinny_gemm(M, N, K):
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(N, K, device=DEV, dtype=torch.bfloat16) * K ** -0.5
+    bias = torch.randn(N, device=DEV, dtype=torch.bfloat16)
+    res = torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    ref = x.float() @ w.float().t()
+    # fp32 sums and one rounding to bf16 (2^-9 of a value at most); GELU adds the 2^-11 of its tanh
+    assert _rel(F.gemm(x, w), ref) < 2 ** -9
+    assert _rel(F.gemm(x, w, bias=bias, aux=res, flags=F.EPI_RESIDUAL), ref + bias.float() + res.float()) < 2 ** -9
+    act = torch.nn.functional.gelu(ref + bias.float(), approximate="tanh")
+    assert _rel(F.gemm(x, w, bias=bias, flags=F.EPI_GELU), act) < 2 ** -8
