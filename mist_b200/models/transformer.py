@@ -21,7 +21,9 @@ import torch.nn as nn
 
 from ..config import AttnMaskType, ModelConfig, PositionEmbeddingType
 from ..modules.layers import ParallelGatedMlp, ParallelMHA, ParallelMLP, get_norm
+from ..ops import decode
 from ..ops import functional as F
+from ..parallel.dist_ops import group_size
 
 
 def _gate_activation(name: str) -> str:
@@ -85,6 +87,10 @@ class ParallelTransformerLayer(nn.Module):
                                    bias1=cfg.mlp_fc1_bias, bias2=cfg.mlp_fc2_bias,
                                    activation=cfg.activation_function,
                                    sequence_parallel=sequence_parallel, **fk)
+
+        # a sequential self-attention block on one rank: what the native decoding step covers
+        self.plain_block = not (self.parallel_block or is_decoder or self.residual_from_norm or self.fp32_residual
+                                or sequence_parallel or group_size(process_group) > 1)
 
     def _drop(self, x):
         if self.hidden_dropout > 0 and self.training:
@@ -181,6 +187,12 @@ class ParallelTransformer(nn.Module):
     def forward(self, hidden, residual=None, encoder_output=None, batch_size=None, attn_mask=None, enc_mask=None):
         if self.input_tensor is not None:
             hidden = self.input_tensor
+        if (self.hooks is None and isinstance(hidden, torch.Tensor) and hidden.dim() == 3 and hidden.shape[1] == 1
+                and not torch.is_grad_enabled() and attn_mask is None and len(self.layers)
+                and getattr(self.layers[0].attn, "inference_params", None) is not None):
+            out = decode.stack_step(self.layers, hidden, residual)
+            if out is not None:
+                return out if self.final_norm is None else self.final_norm(*out)
         n = len(self.layers)
         first_ckpt = n - self.gradient_checkpointing
         hooks = self.hooks

@@ -1,0 +1,122 @@
+"""One decoding step through a stack of plain transformer blocks in one native call (csrc/decode_stack.cu).
+
+:func:`stack_step` looks every block over (structure, types, hooks, dtypes) and hands the pointers of its weights and
+caches to the library, which launches the whole stack.  Anything out of the ordinary -- parallel or cross-attention
+blocks, tensor parallelism, hooks, dropout in training mode, other dtypes, CPU tensors -- is answered with ``None``
+and goes through the modules one by one.
+"""
+from __future__ import annotations
+
+import ctypes
+
+import torch
+
+from . import native
+from .functional import Settings, rope_tables
+from .native import ptr, stream
+
+_PER_BLOCK = 13
+_BF16 = torch.bfloat16
+
+
+def _block(layer, out: list):
+    """Appends the pointers of one block's tensors, in the order of ``Block`` in the native source, without the cache;
+    returns its shape and options, or ``None`` when the block needs the general path."""
+    from ..models.transformer import ParallelTransformerLayer
+    from ..modules import layers as L
+    if type(layer) is not ParallelTransformerLayer or not layer.plain_block:
+        return None
+    m = layer._modules
+    attn, mlp, n1, n2 = m["attn"], m["mlp"], m["norm1"], m["norm2"]
+    gated = type(mlp) is L.ParallelGatedMlp
+    if type(attn) is not L.ParallelMHA or type(n1) is not type(n2) or type(n1) not in (L.LayerNorm, L.RMSNorm):
+        return None
+    if gated:
+        if mlp.gate_act is not None:
+            return None
+    elif type(mlp) is not L.ParallelMLP or not mlp.fused_gelu:
+        return None
+    if layer.hidden_dropout > 0 and layer.training:
+        return None
+    am, mm = attn._modules, mlp._modules
+    wqkv, wo, w1, w2 = am["Wqkv"], am["out_proj"], mm["fc1"], mm["fc2"]
+    for mod in (layer, attn, mlp, n1, n2, wqkv, wo, w1, w2):
+        if mod._forward_hooks or mod._forward_pre_hooks:
+            return None
+    if (type(wqkv) is not L.ColumnParallelLinear or type(w1) is not L.ColumnParallelLinear
+            or type(wo) is not L.RowParallelLinear or type(w2) is not L.RowParallelLinear):
+        return None
+    if attn.rotary_interleaved or attn.rotary_scale_base is not None or n1.eps != n2.eps:
+        return None
+    for mod in (n1, wqkv, wo, n2, w1, w2):
+        ps = mod._parameters
+        for name in ("weight", "bias"):
+            p = ps.get(name)
+            if p is None:
+                out.append(0)
+                continue
+            if p.dtype is not _BF16 or not p.is_contiguous():
+                return None
+            at = p.data_ptr()
+            if at & 15:
+                return None
+            out.append(at)
+    f = w2._parameters["weight"].shape[1]
+    if w1._parameters["weight"].shape[0] != (2 * f if gated else f):
+        return None
+    return (attn.local_heads, attn.local_heads_kv, attn.head_dim, f, gated, type(n1) is L.RMSNorm, n1.eps,
+            attn.rotary_emb_dim, attn.rotary_emb_base)
+
+
+def stack_step(layers, hidden, residual):
+    """``(hidden, residual)`` behind ``layers`` for one new token per sequence (``hidden`` ``[b, 1, h]``), with the
+    caches of the blocks' ``inference_params`` extended by it; ``None`` when the general path is needed."""
+    if (not hidden.is_cuda or hidden.dtype is not _BF16 or torch.is_grad_enabled()
+            or Settings.gemm_backend != "tcgen05"):
+        return None
+    b, s, h = hidden.shape
+    if s != 1 or b > 128 or h % 8 or h > 8192 or not len(layers):
+        return None
+    ptrs, scales, ip, kind, cache_sb = [], [], None, None, 0
+    for layer in layers:
+        k = _block(layer, ptrs)
+        if k is None or (kind is not None and k != kind):
+            return None
+        attn = layer._modules["attn"]
+        mine = attn.__dict__.get("inference_params")
+        if mine is None or (ip is not None and mine is not ip):
+            return None
+        ip, kind = mine, k
+        scales.append(attn.softmax_scale)
+    hq, hk, d, f, gated, rms, eps, rot, base = kind
+    off = ip.seqlen_offset
+    if d % 8 or d > 256 or rot % 16 or f % 64 or hq % hk or off >= ip.max_seqlen:
+        return None
+    caches = [ip.cache_for(layer._modules["attn"].layer_idx, b, hk, d, hidden.dtype, hidden.device) for layer in layers]
+    cache_sb = caches[0].stride(0)
+    for c in caches:
+        if c.dtype is not _BF16 or c.stride() != (cache_sb, 2 * hk * d, hk * d, d, 1) or c.device != hidden.device:
+            return None
+    n = len(caches)
+    table = (ctypes.c_uint64 * (_PER_BLOCK * n))()
+    for i, c in enumerate(caches):
+        table[_PER_BLOCK * i: _PER_BLOCK * (i + 1)] = ptrs[12 * i: 12 * (i + 1)] + [c.data_ptr()]
+    cos = sin = 0
+    if rot:
+        tc, ts = rope_tables(ip.max_seqlen, rot, base, hidden.device)
+        cos, sin = tc.data_ptr() + off * rot * 2, ts.data_ptr() + off * rot * 2      # [position][rot / 2] fp32
+    hidden = hidden.contiguous()
+    if residual is not None:
+        if residual.dtype is not _BF16:
+            return None
+        residual = residual.contiguous()
+    lib = native.kernels()
+    x, r = torch.empty_like(hidden), torch.empty_like(hidden)
+    scratch = torch.empty(lib.mb_decode_stack_scratch(b, h, hq, hk, d, f), dtype=_BF16, device=hidden.device)
+    rc = lib.mb_decode_stack(ptr(hidden), ptr(residual), ptr(x), ptr(r), table, n, ptr(scratch), b, h, hq, hk, d, f,
+                             128 if gated else 2, int(rms), float(eps), (ctypes.c_float * n)(*scales), cos, sin, rot,
+                             off, cache_sb, stream())
+    if rc < 0:
+        raise RuntimeError(f"mb_decode_stack failed with code {rc}")
+    native.launch_count += rc
+    return x, r

@@ -67,3 +67,42 @@ def test_skinny_gemm(M, N, K):
     assert _rel(F.gemm(x, w, bias=bias, aux=res, flags=F.EPI_RESIDUAL), ref + bias.float() + res.float()) < 2 ** -9
     act = torch.nn.functional.gelu(ref + bias.float(), approximate="tanh")
     assert _rel(F.gemm(x, w, bias=bias, flags=F.EPI_GELU), act) < 2 ** -8
+
+
+@pytest.mark.parametrize("model,extra", [("gpt2/1.3b", []), ("llama/1.3b", []), ("llama/1.3b", ["model.num_heads_kv=2"])])
+@pytest.mark.parametrize("b", [1, 5, 40])
+def test_native_decode_step_matches_the_modules(model, extra, b, monkeypatch):
+    """The whole stack in one call against the same step through the modules, over several tokens."""
+    from mist_b200.config import load_config
+    from mist_b200.inference import kv_cache
+    from mist_b200.models.provider import base_model_provider
+    from mist_b200.ops import decode
+    cfg, _ = load_config("config", ["experiment=gpt2-1.3b", f"model={model}", "model.num_hidden_layers=3",
+                                    "model.hidden_size=512", "model.intermediate_size=1408",
+                                    "model.num_attention_heads=8", "model.vocab_size=1024",
+                                    "training.max_sequence_length=64", "strategy.layer_partitions=[3]"] + extra,
+                         check_world_size=False)
+    torch.manual_seed(0)
+    net = base_model_provider(cfg.model, device=torch.device(DEV), dtype=torch.bfloat16).eval()
+    ids = torch.randint(0, 1024, (b, 12), device=DEV)
+
+    def steps():
+        out = []
+        with torch.no_grad(), kv_cache(net, b, 16) as ip:
+            for t in range(12):
+                pos = torch.full((b, 1), t, device=DEV)
+                out.append(net(ids[:, t:t + 1], position_ids=pos).reshape(b, -1).float())
+                ip.seqlen_offset += 1
+            return torch.stack(out), [ip.key_value_memory[i].float() for i in range(3)]
+
+    calls = []
+    native_step = decode.stack_step
+    monkeypatch.setattr(decode, "stack_step", lambda *a: calls.append(native_step(*a)) or calls[-1])
+    got, cache = steps()
+    assert len(calls) == 12 and all(c is not None for c in calls)
+    monkeypatch.setattr(decode, "stack_step", lambda *a: None)
+    want, cache_ref = steps()
+    # three blocks of bf16 roundings at different places (SwiGLU takes unrounded products here)
+    assert _rel(got, want) < 2e-2
+    for a, r in zip(cache, cache_ref):
+        assert _rel(a, r) < 2e-2
