@@ -199,7 +199,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             break;
           }
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             uint32_t sa = smem_u32(smem + s * L::kStageBytes);
             uint32_t sb = sa + L::kABytes;
 #pragma unroll
@@ -214,7 +214,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           }
           __syncwarp();
         }
-        if (ok && lane == 0) mma_commit_pair(&tfull_bar[acc]);
+        if (ok && elect_one()) mma_commit_pair(&tfull_bar[acc]);
         __syncwarp();
       }
     }

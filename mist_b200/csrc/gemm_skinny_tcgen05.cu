@@ -152,7 +152,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         break;
       }
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t sw = smem_u32(smem + s * L::kStage), sx = sw + L::kW;
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k)
@@ -162,7 +162,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       }
       __syncwarp();
     }
-    if (ok && lane == 0) mma_commit(done_bar);
+    if (ok && elect_one()) mma_commit(done_bar);
     __syncwarp();
   } else {
     const int q = warp & 3, r = q * 32 + lane;       // accumulator lane = row of W

@@ -190,7 +190,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           uint32_t sa = smem_u32(smem + s * L::kStageBytes);
           uint32_t sb = sa + L::kABytes;
 #pragma unroll
@@ -205,7 +205,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
         __syncwarp();
       }
-      if (ok && lane == 0) mma_commit(&tfull_bar[acc]);
+      if (ok && elect_one()) mma_commit(&tfull_bar[acc]);
       __syncwarp();
     }
   } else {
