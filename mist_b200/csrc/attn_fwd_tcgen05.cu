@@ -2,17 +2,31 @@
 //
 //   O = softmax(scale * Q K^T + causal mask) V,   LSE = logsumexp per row
 //
-// One CTA owns a 128-row query tile of one (batch, head) and walks the key/value
-// sequence in blocks of BN rows (flash-attention recurrence).  Both GEMMs of a block
-// run on tcgen05.mma with the accumulators in tensor memory:
-//   S  = Q K^T   (A = Q K-major, B = K K-major)      -> TMEM, double buffered
-//   O += P V     (A = P K-major from shared memory, B = V MN-major) -> TMEM
-// Q, K and V tiles arrive by per-CTA TMA (4-D tensor maps over [batch][token][head][d],
-// so a packed qkv projection output is consumed in place; head sizes that are not a
-// multiple of 64, e.g. 80, are zero-filled by the TMA bounds check instead of being
-// padded in memory).  Warps 0-3 do the softmax (one query row per thread, read with
-// tcgen05.ld), warp 4 issues TMA, warp 5 issues the MMAs.  With BN = 64 two CTAs fit
-// on an SM, so one CTA's exponentials overlap the other's tensor-core work.
+// What bounds attention at head size 128 is the exponential unit and the tensor pipe alike (about 1024 cycles
+// each per 128 x 128 block), so both have to run all the time.  One CTA per SM therefore keeps two query tiles
+// in flight: while one tile's exponentials are computed, the other tile's products run.  One MMA warp serves the
+// tiles in turn; with a warp for each, their products interleaved and both tiles' scores arrived together.
+// A tile has two warpgroups, each with 64 of the 128 keys of a block (one row per thread, the row maximum goes
+// through shared memory), so that a scheduler has two warps of a tile to issue from.
+// P never leaves tensor memory: it overwrites S columns of its own half and is the A operand of the P V product.
+// Per tile the order is S(j), softmax, P V(j), S(j+1); P V(j) and S(j+1) are issued back to back, in order, so
+// S(j+1) may overwrite P(j), and the arrival of S(j+1) tells the softmax warps that P V(j) is done, which is when O
+// may be rescaled.  P is handed over in two parts, so half of its product hides behind the other half's exponentials.
+// Measured (cycles): a tile's softmax 2000, its products 1250 with the waits between them, a period of 3400 for both
+// tiles; 32 heads of 128, 8192 tokens, no mask: 1145 -> 961 us (1144 TFLOP/s); 8 x 2048 tokens, 32 heads of 80,
+// causal: 391 -> 257 us; 2 x 256 tokens, 4 heads of 128, causal: 11.2 -> 9.8 us.  The left sides are the kernel
+// before: one tile per CTA, two CTAs per SM, 64 keys per block, P through shared memory.
+//
+// The grid is persistent, one CTA per SM.  The work list is ordered by groups of heads whose keys and values fit
+// L2 together, inside a group by query tile, those with most blocks (causal mask) first, and dealt forwards and
+// backwards in turn, so the CTAs end together.
+//
+// Tensor memory: S0 at column 0, S1 at 128, O0 at 256, O1 at 384; P of keys 64 h ... at S + 64 h.
+// Warps 0-7: softmax and output of tile 0; 8-15: tile 1; 16: K / V loads; 17: MMA; 18: Q loads.
+//
+// Q, K and V tiles arrive by per-CTA TMA (4-D tensor maps over [batch][token][head][d], so a packed qkv projection
+// output is consumed in place; head sizes that are not a multiple of 64, e.g. 80, are zero-filled by the TMA bounds
+// check instead of being padded in memory).
 //
 // Replaces the reference's flash-attention v2 forward, an sm_80 mma.sync kernel
 // (reference: csrc/flash_attn/src/flash_fwd_kernel.h, flash_fwd_launch_template.h:13-28,
@@ -24,8 +38,17 @@ using namespace sm100;
 namespace {
 
 constexpr int BM = 128;
-constexpr int kThreads = 192;
-constexpr int kStages = 2;
+constexpr int BN = 128;
+constexpr int kThreads = 640;
+constexpr int kSlots = 5;                 // ring of K and V tiles in the order K0 V0 K1 V1 ...
+constexpr int kTile = 2 * 128 * 128;      // 128 rows of up to two 64-wide chunks
+constexpr int oRing = 2 * kTile;
+constexpr int oBar = oRing + kSlots * kTile;
+// q_full[2], q_empty[2], full[5], empty[5], s_full[2], p_full[2][2], o_full[2]
+constexpr int kNumBars = 2 + 2 + kSlots + kSlots + 2 + 4 + 2;
+constexpr int oMax = oBar + kNumBars * 8 + 16;      // [tile][half][row] maxima (and, at the end, sums)
+constexpr int kSmem = oMax + 2 * 2 * BM * 4;
+static_assert(kSmem <= 232448, "attention forward: shared memory over the per-CTA limit");
 
 struct AttnParams {
   __nv_bfloat16* o;
@@ -41,22 +64,6 @@ struct AttnParams {
   int* status;
 };
 
-template <int BN>
-struct Smem {
-  // every tile is a stack of [rows][64 bf16] chunks, 128-byte swizzled
-  static constexpr int kQ = 2 * BM * 128;           // up to 2 chunks
-  static constexpr int kKV = 2 * BN * 128;          // one stage of K or V
-  static constexpr int kP = (BN / 64) * BM * 128;
-  static constexpr int oQ = 0;
-  static constexpr int oK = oQ + kQ;
-  static constexpr int oV = oK + kStages * kKV;
-  static constexpr int oP = oV + kStages * kKV;
-  static constexpr int oBar = oP + kP;
-  // q_full, k_full[2], v_full[2], kv_empty[2], s_full[2], s_empty[2], p_full, pv_done, k_empty[2]
-  static constexpr int kNumBars = 1 + 2 + 2 + 2 + 2 + 2 + 1 + 1 + 2;
-  static constexpr int kTotal = oBar + kNumBars * 8 + 16;
-};
-
 __device__ __forceinline__ void report(int* status, int code) {
   if (status) atomicCAS(status, 0, code);
 }
@@ -66,316 +73,428 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&t);
 }
 
-template <int BN>
-__global__ void __launch_bounds__(kThreads, (BN == 64 ? 2 : 1))
+struct Sched {
+  int npairs;      // pairs of query tiles per (batch, head)
+  int bh;          // batch * heads
+  int group;       // (batch, head)s that are walked together
+  int total;
+};
+
+struct Work {
+  int q0[2], nb[2], nbmax, head, batch, sq_b, sk_b, coff;
+};
+
+__device__ __forceinline__ int work_index(int n) {
+  const int c = (n & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  return n * gridDim.x + c;
+}
+
+__device__ __forceinline__ Work work_at(const AttnParams& p, const Sched& s, int t) {
+  Work w;
+  const int per_group = s.group * s.npairs;
+  const int g = t / per_group, r = t - g * per_group;
+  const int gsize = min(s.group, s.bh - g * s.group);
+  const int qi = r / gsize;
+  const int bh = g * s.group + (r - qi * gsize);
+  w.batch = bh / p.nh;
+  w.head = bh - w.batch * p.nh;
+  w.sq_b = p.seqlens_q ? min(p.sq, p.seqlens_q[w.batch]) : p.sq;
+  w.sk_b = p.seqlens_k ? min(p.sk, p.seqlens_k[w.batch]) : p.sk;
+  w.coff = w.sk_b - w.sq_b;
+  w.nbmax = 0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int q0 = (2 * (s.npairs - 1 - qi) + i) * BM;
+    int nb = (q0 < w.sq_b) ? (w.sk_b + BN - 1) / BN : 0;
+    if (p.causal) {
+      const int last = q0 + BM - 1 + w.coff;
+      nb = min(nb, last < 0 ? 0 : last / BN + 1);
+    }
+    w.q0[i] = q0;
+    w.nb[i] = nb;
+    w.nbmax = max(w.nbmax, nb);
+  }
+  return w;
+}
+
+__device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* f, bool wide) {
+  const mb::bf16x8 a = mb::pack8(f), b = mb::pack8(f + 8);
+  if (wide) {
+    const uint32_t* x = reinterpret_cast<const uint32_t*>(&a);
+    const uint32_t* y = reinterpret_cast<const uint32_t*>(&b);
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(dst), "r"(x[0]), "r"(x[1]),
+                 "r"(x[2]), "r"(x[3]), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3])
+                 : "memory");
+  } else {
+    reinterpret_cast<mb::bf16x8*>(dst)[0] = a;
+    reinterpret_cast<mb::bf16x8*>(dst)[1] = b;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
-  using L = Smem<BN>;
+                    const __grid_constant__ CUtensorMap tm_v, const AttnParams p, const Sched sch) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::oBar);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBar);
   uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;
-  uint64_t* v_full = bars + 3;
-  uint64_t* kv_empty = bars + 5;
-  uint64_t* s_full = bars + 7;
-  uint64_t* s_empty = bars + 9;
-  uint64_t* p_full = bars + 11;
-  uint64_t* pv_done = bars + 12;
-  uint64_t* k_empty = bars + 13;   // K stage free as soon as its S MMA has read it (V waits for PV)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::kNumBars);
+  uint64_t* q_empty = bars + 2;
+  uint64_t* full = bars + 4;
+  uint64_t* empty = full + kSlots;
+  uint64_t* s_full = empty + kSlots;
+  uint64_t* p_full = s_full + 2;            // [tile][first, second 32 keys of each half]
+  uint64_t* o_full = p_full + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // heavy (late) query tiles first: under the causal mask they have the most blocks
-  const int qt = gridDim.x - 1 - blockIdx.x;
-  const int head = blockIdx.y;
-  const int batch = blockIdx.z;
-  const int head_kv = head / (p.nh / p.nh_kv);
-  const int q0 = qt * BM;
-  const int sq_b = p.seqlens_q ? min(p.sq, p.seqlens_q[batch]) : p.sq;   // real tokens of this sample
-  const int sk_b = p.seqlens_k ? min(p.sk, p.seqlens_k[batch]) : p.sk;
-  const int coff = sk_b - sq_b;  // causal: key j visible to query i when j <= i + coff
-
-  int nblocks = (q0 < sq_b) ? (sk_b + BN - 1) / BN : 0;   // a tile of padding rows has nothing to attend to
-  if (p.causal) {
-    int last = q0 + BM - 1 + coff;  // last visible key of the tile's last row
-    int nb = last < 0 ? 0 : last / BN + 1;
-    nblocks = min(nblocks, nb);
-  }
 
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need a 1024-byte base
     if (threadIdx.x == 0) report(p.status, MB_ERR_BAD_ARG);
     return;
   }
-
-  constexpr int kTmemCols = (BN == 64) ? 256 : 512;
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&v_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
-      mbar_init(&k_empty[s], 1);
-      mbar_init(&s_full[s], 1);
-      mbar_init(&s_empty[s], 128);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&o_full[i], 1);
+      mbar_init(&p_full[2 * i], 8);           // one arrival of each warp of the tile
+      mbar_init(&p_full[2 * i + 1], 8);
     }
-    mbar_init(p_full, 128);
-    mbar_init(pv_done, 1);
+    for (int i = 0; i < kSlots; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
     fence_barrier_init();
     prefetch_tmap(&tm_q);
     prefetch_tmap(&tm_k);
     prefetch_tmap(&tm_v);
   }
-  if (warp == 4) {
-    tmem_alloc(tmem_slot, kTmemCols);
+  if (warp == 16) {
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base;           // S0 at +0, S1 at +BN
-  const uint32_t tmem_o = tmem_base + 2 * BN;  // O accumulator
+  constexpr uint32_t kChunk = 128 * 128;
 
-  const uint32_t chunk_q = BM * 128, chunk_kv = BN * 128;
-
-  if (warp == 4) {
-    // ----------------------------------------------------------- TMA producer
-    if (lane == 0 && nblocks > 0) {
-      bool ok = true;
-      mbar_expect_tx(q_full, p.nchunks * chunk_q);
-      for (int c = 0; c < p.nchunks; ++c)
-        tma_load_4d(smem + L::oQ + c * chunk_q, &tm_q, q_full, 64 * c, head, q0, batch);
-      for (int j = 0; j < nblocks && ok; ++j) {
-        int st = j % kStages;
-        if (j >= kStages && !mbar_wait(&k_empty[st], ((j / kStages) - 1) & 1)) {
-          report(p.status, MB_ERR_TIMEOUT_EMPTY);
-          ok = false;
-          break;
+  if (warp >= 16) {
+    // 640 threads were launched with 96 registers; 512 * 104 + 128 * 64 is the same sum
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;\n");
+    if (warp == 16) {
+      // ---------------------------------------------------------- K, V producer
+      if (lane == 0) {
+        int n = 0, slot = 0;
+        bool ok = true;
+        auto load = [&](const CUtensorMap* tm, int row, int head_kv, int batch) {
+          if (n >= kSlots && !mbar_wait(&empty[slot], (n / kSlots - 1) & 1)) {
+            report(p.status, MB_ERR_TIMEOUT_EMPTY);
+            ok = false;
+            return;
+          }
+          uint8_t* dst = smem + oRing + slot * kTile;
+          mbar_expect_tx(&full[slot], p.nchunks * kChunk);
+          for (int c = 0; c < p.nchunks; ++c)
+            tma_load_4d(dst + c * kChunk, tm, &full[slot], 64 * c, head_kv, row, batch);
+          ++n;
+          if (++slot == kSlots) slot = 0;
+        };
+        for (int r = 0; ok; ++r) {
+          const int t = work_index(r);
+          if (t >= sch.total) break;
+          const Work w = work_at(p, sch, t);
+          const int head_kv = w.head / (p.nh / p.nh_kv);
+          for (int j = 0; j < w.nbmax && ok; ++j) {
+            load(&tm_k, j * BN, head_kv, w.batch);
+            if (ok) load(&tm_v, j * BN, head_kv, w.batch);
+          }
         }
-        uint8_t* sk_ = smem + L::oK + st * L::kKV;
-        uint8_t* sv_ = smem + L::oV + st * L::kKV;
-        mbar_expect_tx(&k_full[st], p.nchunks * chunk_kv);
-        for (int c = 0; c < p.nchunks; ++c)
-          tma_load_4d(sk_ + c * chunk_kv, &tm_k, &k_full[st], 64 * c, head_kv, j * BN, batch);
-        if (j >= kStages && !mbar_wait(&kv_empty[st], ((j / kStages) - 1) & 1)) {
-          report(p.status, MB_ERR_TIMEOUT_EMPTY);
-          ok = false;
-          break;
-        }
-        mbar_expect_tx(&v_full[st], p.nchunks * chunk_kv);
-        for (int c = 0; c < p.nchunks; ++c)
-          tma_load_4d(sv_ + c * chunk_kv, &tm_v, &v_full[st], 64 * c, head_kv, j * BN, batch);
       }
-    }
-  } else if (warp == 5) {
-    // ------------------------------------------------------------- MMA issuer
-    if (nblocks > 0) {
+    } else if (warp == 18) {
+      // ------------------------------------------------------------- Q producer
+      if (lane == 0) {
+        int cq[2] = {0, 0};
+        bool ok = true;
+        for (int r = 0; ok; ++r) {
+          const int t = work_index(r);
+          if (t >= sch.total) break;
+          const Work w = work_at(p, sch, t);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            if (w.nb[i] == 0 || !ok) continue;
+            if (cq[i] > 0 && !mbar_wait(&q_empty[i], (cq[i] - 1) & 1)) {
+              report(p.status, MB_ERR_TIMEOUT_EMPTY);
+              ok = false;
+              continue;
+            }
+            mbar_expect_tx(&q_full[i], p.nchunks * kChunk);
+            for (int c = 0; c < p.nchunks; ++c)
+              tma_load_4d(smem + i * kTile + c * kChunk, &tm_q, &q_full[i], 64 * c, w.head, w.q0[i], w.batch);
+            ++cq[i];
+          }
+        }
+      }
+    } else if (warp == 17) {
+      // ------------------------------------------------------------- MMA issuer
       const uint32_t idesc_s = make_idesc_bf16(BM, BN, 0, 0);
       const uint32_t idesc_o = make_idesc_bf16(BM, p.d_mma, 0, 1);
-      const uint32_t sq_ = smem_u32(smem + L::oQ);
-      const uint32_t sp_ = smem_u32(smem + L::oP);
+      const uint32_t base = smem_u32(smem);
       const int ksteps = p.d_mma / 16;
+      int cq[2] = {0, 0}, cp[2] = {0, 0};    // Q tiles and P tiles so far
+      int round = 0;
       bool ok = true;
-
-      auto issue_s = [&](int j) -> bool {
-        int st = j % kStages, b = j & 1;
-        if (!mbar_wait(&k_full[st], (j / kStages) & 1)) return false;
-        if (j >= 2 && !mbar_wait(&s_empty[b], ((j >> 1) - 1) & 1)) return false;
-        tc_fence_after();
-        if (lane == 0) {
-          uint32_t sk_ = smem_u32(smem + L::oK + st * L::kKV);
-          for (int kk = 0; kk < ksteps; ++kk) {
-            uint32_t ch = kk >> 2, in = (kk & 3) * 32;
-            uint64_t ad = make_smem_desc_sw128(sq_ + ch * chunk_q + in, 16, 1024);
-            uint64_t bd = make_smem_desc_sw128(sk_ + ch * chunk_kv + in, 16, 1024);
-            mma_f16_ss(tmem_s + b * BN, ad, bd, idesc_s, kk != 0 ? 1u : 0u);
-          }
-          mma_commit(&k_empty[st]);
-          mma_commit(&s_full[b]);
+      auto wait = [&](uint64_t* bar, int phase, int code) -> bool {
+        if (ok && !mbar_wait(bar, phase & 1)) {
+          report(p.status, code);
+          ok = false;
         }
-        __syncwarp();
-        return true;
+        return ok;
       };
-
-      if (!mbar_wait(q_full, 0)) { report(p.status, MB_ERR_TIMEOUT_FULL); ok = false; }
-      if (ok && !issue_s(0)) { report(p.status, MB_ERR_TIMEOUT_FULL); ok = false; }
-      for (int j = 0; j < nblocks && ok; ++j) {
-        if (j + 1 < nblocks && !issue_s(j + 1)) {
-          report(p.status, MB_ERR_TIMEOUT_FULL);
-          ok = false;
-          break;
+      // The next item of the list with a block to compute; nbmax = 0 at the end of the list.
+      auto next_work = [&]() -> Work {
+        for (;;) {
+          const int t = work_index(round++);
+          Work w;
+          w.nbmax = 0;
+          if (t < sch.total) w = work_at(p, sch, t);
+          if (t >= sch.total || w.nbmax > 0) return w;
         }
-        int st = j % kStages;
-        if (!mbar_wait(p_full, j & 1) || !mbar_wait(&v_full[st], (j / kStages) & 1)) {
-          report(p.status, MB_ERR_TIMEOUT_TMEM);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        if (lane == 0) {
-          uint32_t sv_ = smem_u32(smem + L::oV + st * L::kKV);
+      };
+      // Next slot of the ring, once it is full.
+      int slot = 0, lap = 0;
+      auto take_slot = [&]() -> int {
+        const int at = slot;
+        wait(&full[at], lap, MB_ERR_TIMEOUT_FULL);
+        if (++slot == kSlots) { slot = 0; lap ^= 1; }
+        return at;
+      };
+      // S(j) = Q K(j)^T of tile i; tile 1 comes last and releases the slot
+      auto issue_s = [&](int i, int at, bool active, bool last) {
+        if (elect_one()) {
+          if (active) {
+            const uint64_t dq = make_smem_desc_sw128(base + i * kTile, 16, 1024);
+            const uint64_t dk = make_smem_desc_sw128(base + oRing + at * kTile, 16, 1024);
 #pragma unroll
-          for (int kk = 0; kk < BN / 16; ++kk) {
-            uint32_t ch = kk >> 2, in = (kk & 3) * 32;
-            uint64_t ad = make_smem_desc_sw128(sp_ + ch * chunk_q + in, 16, 1024);
-            // V: [kv rows][64-wide d atoms]; 16 kv rows = 2048 B, next d atom = chunk_kv
-            uint64_t bd = make_smem_desc_sw128(sv_ + kk * 2048, chunk_kv, 1024);
-            mma_f16_ss(tmem_o, ad, bd, idesc_o, (j | kk) != 0 ? 1u : 0u);
+            for (int kk = 0; kk < 8; ++kk) {
+              const uint32_t off = ((kk >> 2) * kChunk + (kk & 3) * 32) >> 4;
+              if (kk < ksteps) mma_f16_ss(tmem_base + i * 128, dq + off, dk + off, idesc_s, kk != 0 ? 1u : 0u);
+            }
+            mma_commit(&s_full[i]);
+            if (last) mma_commit(&q_empty[i]);
           }
-          mma_commit(&kv_empty[st]);
-          mma_commit(pv_done);
+          if (i == 1) mma_commit(&empty[at]);
         }
         __syncwarp();
+      };
+      // the first S of an item also waits for its Q tile
+      auto first_s = [&](const Work& w, int i, int at) {
+        if (w.nb[i] > 0) wait(&q_full[i], cq[i]++, MB_ERR_TIMEOUT_FULL);
+        if (!ok) return;
+        tc_fence_after();
+        issue_s(i, at, w.nb[i] > 0, w.nb[i] == 1);
+      };
+      Work cur = next_work();
+      if (cur.nbmax > 0) {
+        const int at = take_slot();
+        first_s(cur, 0, at);
+        first_s(cur, 1, at);
+      }
+      while (ok && cur.nbmax > 0) {
+        const Work nxt = next_work();
+        for (int j = 0; j < cur.nbmax && ok; ++j) {
+          const bool inside = j + 1 < cur.nbmax;
+          const int at_v = take_slot();
+          int at_k = 0;
+          if (inside || nxt.nbmax > 0) at_k = take_slot();
+          if (!ok) break;
+          const uint64_t dv = make_smem_desc_sw128(base + oRing + at_v * kTile, kChunk, 1024);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int active = cur.nb[i];
+            if (j < active) {
+              const uint32_t t_s = tmem_base + i * 128, t_o = tmem_base + 256 + i * 128;
+#pragma unroll
+              for (int part = 0; part < 2; ++part) {
+                if (!wait(&p_full[2 * i + part], cp[i], MB_ERR_TIMEOUT_TMEM)) break;
+                tc_fence_after();
+                if (elect_one()) {
+                  // part 0: the first 32 keys of both halves; 16 keys are 8 columns of P and 2048 B of V
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) {
+                    const int kk = 4 * (u >> 1) + 2 * part + (u & 1);
+                    mma_f16_ts(t_o, t_s + 64 * (kk >> 2) + 8 * (kk & 3), dv + kk * (2048 >> 4), idesc_o,
+                               (j | kk) != 0 ? 1u : 0u);
+                  }
+                  if (part == 1 && j == active - 1) mma_commit(&o_full[i]);
+                }
+                __syncwarp();
+              }
+              if (!ok) break;
+              ++cp[i];
+            }
+            if (i == 1 && elect_one()) mma_commit(&empty[at_v]);
+            __syncwarp();
+            if (inside) issue_s(i, at_k, j + 1 < active, j + 2 == active);
+            else if (nxt.nbmax > 0) first_s(nxt, i, at_k);
+          }
+        }
+        cur = nxt;
       }
     }
   } else {
-    // ---------------------------------------------------------------- softmax
-    const int r = threadIdx.x;  // row of the tile == TMEM lane
-    const int qi = q0 + r;
-    const uint32_t lane_off = static_cast<uint32_t>(warp * 32) << 16;
-    float m_run = -INFINITY, l_run = 0.f;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;\n");
+    // ------------------------------------------------------- softmax and output
+    const int i = warp >> 3;          // query tile
+    const int h = (warp >> 2) & 1;    // half of the keys of a block, and of the output's columns
+    const int r = threadIdx.x & 127;  // row of the tile == TMEM lane
+    const int pair_bar = 1 + 4 * i + (warp & 3);      // named barrier of the two warps that share these rows
+    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t t_s = tmem_base + i * 128 + 64 * h + lane_off, t_o = tmem_base + 256 + i * 128 + lane_off;
+    float* s_max = reinterpret_cast<float*>(smem + oMax) + i * 2 * BM + r;    // [half]
+    const mb::f32x2 scale2 = mb::pack_f32x2(p.scale_log2, p.scale_log2);
+    const bool wide = ((reinterpret_cast<uintptr_t>(p.o) & 31) | ((p.o_tok_stride | p.o_head_stride |
+                       p.o_batch_stride) & 15)) == 0;
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory"); };
+    int cs = 0, co = 0;               // S tiles and O tiles so far
     bool ok = true;
-    uint8_t* sp_ = smem + L::oP;
+    for (int rnd = 0; ok; ++rnd) {
+      const int t = work_index(rnd);
+      if (t >= sch.total) break;
+      const Work w = work_at(p, sch, t);
+      const int q0 = i ? w.q0[1] : w.q0[0], nb = i ? w.nb[1] : w.nb[0];
+      const int qi = q0 + r;
+      const int vis = (p.causal ? min(w.sk_b - 1, qi + w.coff) : w.sk_b - 1) - 64 * h;   // last visible key of the row
+      const int vis_tile = p.causal ? min(w.sk_b - 1, q0 + w.coff) : w.sk_b - 1;         // of the tile's first row
+      float m_run = -INFINITY, l_run = 0.f;
 
-    for (int j = 0; j < nblocks && ok; ++j) {
-      const int b = j & 1;
-      if (!mbar_wait(&s_full[b], (j >> 1) & 1)) {
-        report(p.status, MB_ERR_TIMEOUT_TMEM);
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      uint32_t sr[BN];
-#pragma unroll
-      for (int c = 0; c < BN / 32; ++c) tmem_ld32(tmem_s + b * BN + c * 32 + lane_off, sr + 32 * c);
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(&s_empty[b]);
-
-      const int kv0 = j * BN;
-      const int vis = p.causal ? min(sk_b - 1, qi + coff) : sk_b - 1;  // last visible key
-      // Only tiles that touch the diagonal or the end of the keys need the mask; the test is the
-      // same for every thread of the CTA (first row of the tile has the smallest horizon).
-      const int vis_tile = p.causal ? min(sk_b - 1, q0 + coff) : sk_b - 1;
-      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-      if (kv0 + BN - 1 > vis_tile) {
-#pragma unroll
-        for (int i = 0; i < BN; i += 4) {
-          float v0 = (kv0 + i <= vis) ? __uint_as_float(sr[i]) : -INFINITY;
-          float v1 = (kv0 + i + 1 <= vis) ? __uint_as_float(sr[i + 1]) : -INFINITY;
-          float v2 = (kv0 + i + 2 <= vis) ? __uint_as_float(sr[i + 2]) : -INFINITY;
-          float v3 = (kv0 + i + 3 <= vis) ? __uint_as_float(sr[i + 3]) : -INFINITY;
-          sr[i] = __float_as_uint(v0); sr[i + 1] = __float_as_uint(v1);
-          sr[i + 2] = __float_as_uint(v2); sr[i + 3] = __float_as_uint(v3);
-          mx0 = fmaxf(mx0, v0); mx1 = fmaxf(mx1, v1); mx2 = fmaxf(mx2, v2); mx3 = fmaxf(mx3, v3);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < BN; i += 4) {
-          mx0 = fmaxf(mx0, __uint_as_float(sr[i]));
-          mx1 = fmaxf(mx1, __uint_as_float(sr[i + 1]));
-          mx2 = fmaxf(mx2, __uint_as_float(sr[i + 2]));
-          mx3 = fmaxf(mx3, __uint_as_float(sr[i + 3]));
-        }
-      }
-      // raw scores; the softmax scale (> 0, so maxima commute with it) is folded into the FFMA below
-      const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2;
-      // Lazy rescaling: keep the old reference maximum unless the new one is much
-      // larger; probabilities then stay below 2^8, harmless in fp32 / bf16.
-      const float m_new = fmaxf(m_run, mx);
-      const float m_use = (m_new - m_run > 8.f || m_run == -INFINITY) ? m_new : m_run;
-      const float alpha = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_use);
-      const float m_neg = (m_use == -INFINITY) ? 0.f : -m_use;
-      float sum0 = 0.f, sum1 = 0.f;
-      uint32_t pk[BN / 2];
-#pragma unroll
-      for (int i = 0; i < BN; i += 2) {
-        const float xa = fmaf(__uint_as_float(sr[i]), p.scale_log2, m_neg);
-        const float xc = fmaf(__uint_as_float(sr[i + 1]), p.scale_log2, m_neg);
-        const float a = mb::fast_exp2(xa);
-        const float c = mb::fast_exp2(xc);
-        sum0 += a;
-        sum1 += c;
-        pk[i >> 1] = pack_bf16x2(a, c);
-      }
-      const float sum = sum0 + sum1;
-      l_run = l_run * alpha + sum;
-      m_run = m_use;
-
-      if (j > 0) {
-        if (!mbar_wait(pv_done, (j - 1) & 1)) {
+      for (int j = 0; j < nb; ++j) {
+        if (!mbar_wait(&s_full[i], cs & 1)) {
           report(p.status, MB_ERR_TIMEOUT_TMEM);
           ok = false;
           break;
         }
         tc_fence_after();
-      }
-      // P tile -> shared memory in the swizzled K-major layout the MMA reads
+        uint32_t sr[64];
+        tmem_ld32(t_s, sr);
+        tmem_ld32(t_s + 32, sr + 32);
+        tmem_ld_wait();
+        if (j * BN + BN - 1 > vis_tile) {
+          const int lim = vis - j * BN;      // last visible column
 #pragma unroll
-      for (int g = 0; g < BN / 8; ++g) {
-        uint32_t ch = g >> 3, gg = g & 7;
-        uint4 val = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
-        *reinterpret_cast<uint4*>(sp_ + ch * chunk_q + r * 128 + ((gg ^ (r & 7)) << 4)) = val;
-      }
-      // Rescale the running output when this warp's reference maxima moved.
-      const bool need = (j > 0) && (alpha != 1.f);
-      if (__any_sync(0xffffffffu, need)) {
-        for (int c = 0; c < p.d_mma / 16; ++c) {
-          uint32_t o[16];
-          tmem_ld16(tmem_o + c * 16 + lane_off, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st16(tmem_o + c * 16 + lane_off, o);
+          for (int c = 0; c < 64; ++c) sr[c] = (c <= lim) ? sr[c] : 0xff800000u;
         }
-        tmem_st_wait();
+        float mx[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mx[u] = fmaxf(__uint_as_float(sr[u]), __uint_as_float(sr[4 + u]));
+#pragma unroll
+        for (int c = 8; c < 64; c += 8) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            mx[u] = fmaxf(mx[u], fmaxf(__uint_as_float(sr[c + u]), __uint_as_float(sr[c + 4 + u])));
+        }
+        // the next write comes after the next s_full, that is after the other half's arrival on p_full, below its read
+        const float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        s_max[h * BM] = mine;
+        pair_sync();
+        ++cs;
+        // raw scores; the softmax scale (> 0, so maxima commute with it) is folded into the FFMA below
+        const float mxs = fmaxf(mine, s_max[(h ^ 1) * BM]) * p.scale_log2;
+        // Lazy rescaling: keep the old reference maximum unless the new one is much larger; probabilities then
+        // stay below 2^8, harmless in fp32 / bf16.
+        const float m_new = fmaxf(m_run, mxs);
+        const float m_use = (m_new - m_run > 8.f || m_run == -INFINITY) ? m_new : m_run;
+        const float alpha = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_use);
+        const float m_neg = (m_use == -INFINITY) ? 0.f : -m_use;
+        // S(j) is complete, so P V(j-1), issued before it, is too: O may be rescaled, each half its columns
+        if (__any_sync(0xffffffffu, j > 0 && alpha != 1.f)) {      // before the arrivals on p_full, which P V waits for
+          for (int c = 16 * h; c < p.d_mma; c += 32) {
+            uint32_t o[16];
+            tmem_ld16(t_o + c, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int u = 0; u < 16; ++u) o[u] = __float_as_uint(__uint_as_float(o[u]) * alpha);
+            tmem_st16(t_o + c, o);
+          }
+        }
+        const mb::f32x2 m2 = mb::pack_f32x2(m_neg, m_neg);
+        mb::f32x2 sum0 = 0, sum1 = 0;
+        // P in two parts, so that the first half of its product runs beside the second half of the exponentials
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int c = 0; c < 32; c += 4) {
+            const uint32_t* s4 = sr + 32 * part + c;
+            const float2 xa = mb::unpack_f32x2(
+                mb::fma_f32x2(mb::pack_f32x2(__uint_as_float(s4[0]), __uint_as_float(s4[1])), scale2, m2));
+            const float2 xb = mb::unpack_f32x2(
+                mb::fma_f32x2(mb::pack_f32x2(__uint_as_float(s4[2]), __uint_as_float(s4[3])), scale2, m2));
+            const float a0 = mb::fast_exp2(xa.x), a1 = mb::fast_exp2(xa.y);
+            const float b0 = mb::fast_exp2(xb.x), b1 = mb::fast_exp2(xb.y);
+            sum0 = mb::add_f32x2(sum0, mb::pack_f32x2(a0, a1));
+            sum1 = mb::add_f32x2(sum1, mb::pack_f32x2(b0, b1));
+            pk[c >> 1] = pack_bf16x2(a0, a1);
+            pk[(c >> 1) + 1] = pack_bf16x2(b0, b1);
+          }
+          tmem_st16(t_s + 16 * part, pk);
+          tmem_st_wait();
+          tc_fence_before();
+          mbar_arrive_warp(&p_full[2 * i + part]);
+        }
+        const float2 sum = mb::unpack_f32x2(mb::add_f32x2(sum0, sum1));
+        l_run = l_run * alpha + (sum.x + sum.y);
+        m_run = m_use;
       }
-      fence_async_smem();
-      tc_fence_before();
-      mbar_arrive(p_full);
-    }
+      if (!ok) break;
 
-    if (ok && nblocks > 0) {
-      if (!mbar_wait(pv_done, (nblocks - 1) & 1)) {
-        report(p.status, MB_ERR_TIMEOUT_TMEM);
-        ok = false;
+      if (nb > 0) {
+        if (!mbar_wait(&o_full[i], co & 1)) {
+          report(p.status, MB_ERR_TIMEOUT_TMEM);
+          ok = false;
+          break;
+        }
+        ++co;
+        tc_fence_after();
       }
-    }
-    if (ok) {
-      tc_fence_after();
-      const bool real_row = qi < sq_b;
+      // the other half's share of the row sum (the last block's P V is done: both halves have read the maxima)
+      s_max[h * BM] = l_run;
+      pair_sync();
+      l_run = s_max[0] + s_max[BM];
+      pair_sync();
+      const bool real_row = qi < w.sq_b;
       const float inv = (real_row && l_run > 0.f) ? 1.f / l_run : 0.f;
-      __nv_bfloat16* orow = p.o + batch * p.o_batch_stride + static_cast<long>(qi) * p.o_tok_stride +
-                            static_cast<long>(head) * p.o_head_stride;
-      for (int c = 0; c < p.d_mma / 16; ++c) {
+      __nv_bfloat16* orow = p.o + w.batch * p.o_batch_stride + static_cast<long>(qi) * p.o_tok_stride +
+                            static_cast<long>(w.head) * p.o_head_stride;
+      for (int c = 16 * h; c < p.d; c += 32) {
         uint32_t o[16];
-        if (nblocks > 0) {
-          tmem_ld16(tmem_o + c * 16 + lane_off, o);
+        if (nb > 0) {
+          tmem_ld16(t_o + c, o);
           tmem_ld_wait();
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = 0;
+          for (int u = 0; u < 16; ++u) o[u] = 0;
         }
-        if (qi < p.sq && c * 16 < p.d) {
+        if (qi < p.sq) {
           float f[16];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(o[i]) * inv;
-          *reinterpret_cast<mb::bf16x8*>(orow + c * 16) = mb::pack8(f);
-          *reinterpret_cast<mb::bf16x8*>(orow + c * 16 + 8) = mb::pack8(f + 8);
+          for (int u = 0; u < 16; ++u) f[u] = __uint_as_float(o[u]) * inv;
+          store16(orow + c, f, wide);
         }
       }
-      if (qi < p.sq)
-        p.lse[(static_cast<long>(batch) * p.nh + head) * p.sq + qi] =
+      tc_fence_before();
+      if (h == 0 && qi < p.sq)
+        p.lse[(static_cast<long>(w.batch) * p.nh + w.head) * p.sq + qi] =
             (real_row && l_run > 0.f) ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == 16) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -429,7 +548,7 @@ MB_API int* mb_status_device_ptr();
 MB_API int mb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int batch,
                        int sq, int sk, int nh, int nh_kv, int d, long q_bs, long q_ts, long q_hs,
                        long k_bs, long k_ts, long k_hs, long v_bs, long v_ts, long v_hs, long o_bs,
-                       long o_ts, long o_hs, float scale, int causal, int block_n, const int* seqlens_q,
+                       long o_ts, long o_hs, float scale, int causal, const int* seqlens_q,
                        const int* seqlens_k, cudaStream_t stream) {
   if (d % 16 || d > 128 || d < 16 || nh % nh_kv) return -1;
   if ((q_ts | q_hs | q_bs | k_ts | k_hs | k_bs | v_ts | v_hs | v_bs | o_ts | o_hs | o_bs) & 7) return -1;
@@ -437,11 +556,12 @@ MB_API int mb_attn_fwd(const void* q, const void* k, const void* v, void* o, flo
        reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(o)) & 15)
     return -1;
   if (batch == 0 || sq == 0) return 0;
-  const int bn = (block_n == 128) ? 128 : 64;
+  const long pairs = (sq + 2 * BM - 1) / (2 * BM), units = pairs * nh * batch;
+  if (units > 0x3fffffff) return -1;
   CUtensorMap tq, tk, tv;
   if (!make_map(&tq, q, batch, sq, nh, d, q_bs, q_ts, q_hs, BM)) return -2;
-  if (!make_map(&tk, k, batch, sk, nh_kv, d, k_bs, k_ts, k_hs, bn)) return -2;
-  if (!make_map(&tv, v, batch, sk, nh_kv, d, v_bs, v_ts, v_hs, bn)) return -2;
+  if (!make_map(&tk, k, batch, sk, nh_kv, d, k_bs, k_ts, k_hs, BN)) return -2;
+  if (!make_map(&tv, v, batch, sk, nh_kv, d, v_bs, v_ts, v_hs, BN)) return -2;
   AttnParams p;
   p.o = reinterpret_cast<__nv_bfloat16*>(o);
   p.lse = lse;
@@ -454,20 +574,21 @@ MB_API int mb_attn_fwd(const void* q, const void* k, const void* v, void* o, flo
   p.seqlens_q = seqlens_q;
   p.seqlens_k = seqlens_k;
   p.status = mb_status_device_ptr();
-  dim3 grid((sq + BM - 1) / BM, nh, batch);
-#define MB_ATTN_LAUNCH(BN_)                                                                        \
-  do {                                                                                             \
-    auto kern = attn_fwd_kernel<BN_>;                                                              \
-    static bool cfg = false;                                                                       \
-    if (!cfg) {                                                                                    \
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
-                               Smem<BN_>::kTotal) != cudaSuccess) return -3;                       \
-      cfg = true;                                                                                  \
-    }                                                                                              \
-    kern<<<grid, kThreads, Smem<BN_>::kTotal, stream>>>(tq, tk, tv, p);                            \
-  } while (0)
-  if (bn == 64) MB_ATTN_LAUNCH(64);
-  else MB_ATTN_LAUNCH(128);
-#undef MB_ATTN_LAUNCH
+  static bool cfg = false;
+  if (!cfg) {
+    if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
+      return -3;
+    cfg = true;
+  }
+  Sched sch;
+  sch.npairs = static_cast<int>(pairs);
+  sch.bh = nh * batch;
+  // heads whose keys and values take about a third of L2 together, at least one key / value head
+  const long kv_bytes = 4l * sk * d;
+  const long kv_heads = kv_bytes > 0 ? (40l << 20) / kv_bytes : 1;
+  const long group = (kv_heads < 1 ? 1 : kv_heads) * (nh / nh_kv);
+  sch.group = static_cast<int>(group < sch.bh ? group : sch.bh);
+  sch.total = static_cast<int>(units);
+  attn_fwd_kernel<<<units < 148 ? static_cast<int>(units) : 148, kThreads, kSmem, stream>>>(tq, tk, tv, p, sch);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -47,10 +47,8 @@ class Settings:
     """Process-wide kernel selection switches."""
     gemm_backend = "tcgen05"      # "tcgen05" (ours) | "cublas" (library, A/B baseline)
     attn_backend = "tcgen05"      # "tcgen05" (ours) | "sdpa" (library, A/B baseline)
-    attn_block_n = 64
-    # Backward kernel that overlaps the next block's S / dP products with the current block's softmax
-    # (6 % faster than the unpipelined kernel at head sizes 80 and 128; MIST_B200_ATTN_BWD_PIPELINED=0
-    # selects the unpipelined one).
+    # Backward kernel on 128 x 128 blocks that overlaps the next block's S / dP products with the current block's
+    # softmax; MIST_B200_ATTN_BWD_PIPELINED=0 selects the one that finishes a 64-row query block before the next.
     attn_bwd_pipelined = os.environ.get("MIST_B200_ATTN_BWD_PIPELINED", "1") != "0"
     gemm_max_ctas = 0             # >0 leaves SMs free for a concurrent communication kernel
     gemm_pair = True              # large GEMMs on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2)
@@ -791,7 +789,8 @@ def _select_variant(setter: str, want: int):
 
 def attn_fwd(q, k, v, scale, causal, block_n=None, seqlens_q=None, seqlens_k=None):
     """Forward only: returns (o [b,sq,nh,d], lse [b,nh,sq] fp32).  ``seqlens_q`` / ``seqlens_k``: int32
-    device tensors ``[b]`` with the number of real tokens of each sample of a right-padded batch."""
+    device tensors ``[b]`` with the number of real tokens of each sample of a right-padded batch.
+    ``block_n`` has no effect (the kernel has one block size); it is accepted for callers that pass it."""
     if not use_native(q):
         return _ref_attention(q, k, v, scale, causal, seqlens_q, seqlens_k)
     b, sq, nh, d = q.shape
@@ -802,7 +801,7 @@ def attn_fwd(q, k, v, scale, causal, block_n=None, seqlens_q=None, seqlens_k=Non
     call("mb_attn_fwd", ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), b, sq, sk, nh, nkv, d,
          q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
          v.stride(0), v.stride(1), v.stride(2), o.stride(0), o.stride(1), o.stride(2),
-         float(scale), int(causal), block_n or Settings.attn_block_n, ptr(seqlens_q), ptr(seqlens_k), stream())
+         float(scale), int(causal), ptr(seqlens_q), ptr(seqlens_k), stream())
     return o, lse
 
 

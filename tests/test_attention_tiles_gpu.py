@@ -63,7 +63,7 @@ def test_block_kernels_at_tile_edges(b, sq, sk, nh, nkv, d, causal):
     scale = 1 / math.sqrt(d)
     leaves = [t.double().requires_grad_(True) for t in (q, k, v)]
     o_ref, lse_ref = _exact(*leaves, scale, causal)
-    o, lse = F.attn_fwd(q, k, v, scale, causal, block_n=256)
+    o, lse = F.attn_fwd(q, k, v, scale, causal)
     _close(o, o_ref)
     seen = torch.isfinite(lse_ref)
     assert torch.equal(torch.isfinite(lse), seen)
@@ -85,7 +85,7 @@ def test_block_kernels_on_padded_batches(d, causal):
     scale = 1 / math.sqrt(d)
     leaves = [t.double().requires_grad_(True) for t in (q, k, v)]
     o_ref, _ = _exact(*leaves, scale, causal, lens, lens)
-    o, lse = F.attn_fwd(q, k, v, scale, causal, block_n=256, seqlens_q=lens, seqlens_k=lens)
+    o, lse = F.attn_fwd(q, k, v, scale, causal, seqlens_q=lens, seqlens_k=lens)
     _close(o, o_ref)
     grads = attention_bwd.backward(g, q, k, v, o, lse, scale, causal, seqlens=(lens, lens))
     native.check_status()
