@@ -12,7 +12,9 @@
 // 128 B a cycle.  128 query rows per block instead of 64 are what makes the two meet: a 128 x 64 product takes its
 // operands from shared memory at two thirds of the tensor rate.  The MMA warp issues S^T of block i+1 before it
 // waits for dS^T of block i, so the exponentials run beside the dQ, dK products of the block before.
-// dQ is added to an fp32 accumulator with TMA reduces by a warpgroup of its own.
+// dQ is added to an fp32 accumulator with TMA reduces by a warpgroup of its own: about 850 cycles per 128 x 32 values,
+// which at head size 128 is as long as the block's products.  (Untiled bulk reduces of the same bytes into a contiguous
+// accumulator took 1150.)
 //
 // Tensor memory (columns): head size up to 80: S^T 0, dP^T 128, dQ 256, dV 336, dK 416; above, dQ has no columns of
 // its own and takes dP^T's: S^T 0, dP^T / dQ 128, dV 256, dK 384.
@@ -21,7 +23,7 @@
 // by key block (under the causal mask the first blocks are the longest), dealt forwards and backwards in turn.
 //
 // Warps 0-15: softmax (warpgroup w: query columns 32 w ... of the block) and dK / dV output; 16-19: dQ; 20: loads;
-// 21: MMA.  Barriers (one phase per block i unless noted; a phase is never entered twice because every arrival for
+// 21: MMA; 22: LSE and delta (in the softmax warps their latency, 1300 cycles, was part of every block).  Barriers (one phase per block i unless noted; a phase is never entered twice because every arrival for
 // block i+1 follows a wait that needs block i's phase):
 //   q_full/q_empty[2], do_full/do_empty   loads of Q and dO
 //   k_full, k_empty, v_full, v_empty      one phase per work item
@@ -30,6 +32,7 @@
 //   ds_full, ds_empty  softmax <-> MMA    dS^T is in shared memory (and dP^T in registers) / has been read
 //   dq_full, dq_empty  MMA <-> dQ warps   dQ is complete / is in registers
 //   fin_full           MMA -> softmax     one phase per work item: dV, dK are complete
+//   vec_full/vec_empty[2]                 LSE and delta of the block's queries
 #pragma once
 
 namespace wide {
@@ -41,7 +44,7 @@ constexpr int kDqChunk = BB * 128;        // [128 q][32 fp32]
 constexpr int oK = 0, oV = kTile, oQ = 2 * kTile, oDO = 4 * kTile, oDS = 5 * kTile, oDQ = 6 * kTile;
 constexpr int oVec = oDQ + 2 * kDqChunk;  // -LSE*log2(e) and -delta of two query blocks
 constexpr int oBar = oVec + 2 * 2 * BB * 4;
-constexpr int kNumBars = 4 + 2 + 4 + 2 + 1 + 2 + 2 + 1;
+constexpr int kNumBars = 4 + 4 + 2 + 2 + 1 + 2 + 2 + 1 + 4;
 constexpr int kSmem = oBar + kNumBars * 8 + 16;
 static_assert(kSmem <= 232448, "attention backward: shared memory over the per-CTA limit");
 
@@ -126,6 +129,8 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint64_t* dq_full = bars + 15;
   uint64_t* dq_empty = bars + 16;
   uint64_t* fin_full = bars + 17;
+  uint64_t* vec_full = bars + 18;
+  uint64_t* vec_empty = bars + 20;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
 
   const int warp = threadIdx.x >> 5;
@@ -138,7 +143,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (threadIdx.x == 0) {
     for (int i = 0; i < kNumBars; ++i) {
       const uint64_t* b = bars + i;
-      mbar_init(bars + i, (b == p_full || b == ds_full) ? 16 : (b == dq_empty ? 4 : 1));   // arrivals of warps
+      mbar_init(bars + i, (b == p_full || b == ds_full || b >= vec_empty) ? 16 : (b == dq_empty ? 4 : 1));   // warps
     }
     fence_barrier_init();
     prefetch_tmap(&tm_q);
@@ -196,6 +201,41 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             if (++i == w.per_head) { i = 0; ++hh; }
           }
           ++items;
+        }
+      }
+    } else if (warp == 22) {
+      // ------------------------------------------- LSE and delta of every query block
+      float* s_vec = reinterpret_cast<float*>(smem + oVec);
+      int n = 0;
+      bool ok = true;
+      for (int r = 0; ok; ++r) {
+        const int t = work_index(r);
+        if (t >= sch.total) break;
+        const Work w = work_at(p, sch, t);
+        int hh = 0, i = 0;
+        for (int it = 0; it < w.n_iter; ++it, ++n) {
+          const long row = (static_cast<long>(w.batch) * p.nh + w.unit * sch.unit_heads + hh) * p.sq;
+          const int q = (w.i_start + i) * BB + lane;
+          float lse[4], delta[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const bool in = q + 32 * u < w.sq_b;
+            lse[u] = in ? p.lse[row + q + 32 * u] : 0.f;
+            delta[u] = in ? p.delta[row + q + 32 * u] : 0.f;
+          }
+          if (n >= 2 && !mbar_wait(&vec_empty[n & 1], ((n >> 1) - 1) & 1)) {
+            report(p.status, MB_ERR_TIMEOUT_EMPTY);
+            ok = false;
+            break;
+          }
+          float* dst = s_vec + (n & 1) * 2 * BB + lane;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            dst[32 * u] = lse[u] * -1.4426950408889634f;
+            dst[BB + 32 * u] = -delta[u];
+          }
+          mbar_arrive_warp(&vec_full[n & 1]);
+          if (++i == w.per_head) { i = 0; ++hh; }
         }
       }
     } else if (warp == 21) {
@@ -269,13 +309,17 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           __syncwarp();
           if (next) issue_s(n + 1);
           if (!wait(ds_full, n, MB_ERR_TIMEOUT_TMEM)) break;
-          if (!kAlias) {
-            if (next) issue_dp(n + 1, it + 2 == w.n_iter);
-            if (n > 0 && !wait(dq_empty, n - 1, MB_ERR_TIMEOUT_TMEM)) break;
-          }
-          if (!ok) break;
           tc_fence_after();
-          if (elect_one()) {
+          auto issue_dk = [&]() {
+            const uint64_t d_ds_k = make_smem_desc_sw128(base + oDS, 16, 1024);
+            const uint64_t d_q_mn = make_smem_desc_sw128(base + oQ + (n & 1) * kTile, kChunk, 1024);
+#pragma unroll
+            for (int kk = 0; kk < BB / 16; ++kk)
+              mma_f16_ss(t_dk, d_ds_k + (((kk >> 2) * kChunk + (kk & 3) * 32) >> 4), d_q_mn + kk * (2048 >> 4), idesc_dkv,
+                         (it | kk) != 0);
+            mma_commit(&q_empty[n & 1]);
+          };
+          auto issue_dq = [&]() {
             const uint64_t d_ds_mn = make_smem_desc_sw128(base + oDS, kChunk, 1024);
             const uint64_t d_k_mn = make_smem_desc_sw128(base + oK, kChunk, 1024);
 #pragma unroll
@@ -283,18 +327,30 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               mma_f16_ss(t_dq, d_ds_mn + kk * (2048 >> 4), d_k_mn + kk * (2048 >> 4), idesc_dq, kk != 0);
             mma_commit(dq_full);
             if (!next) mma_commit(k_empty);
-            const uint64_t d_ds_k = make_smem_desc_sw128(base + oDS, 16, 1024);
-            const uint64_t d_q_mn = make_smem_desc_sw128(base + oQ + (n & 1) * kTile, kChunk, 1024);
-#pragma unroll
-            for (int kk = 0; kk < BB / 16; ++kk)
-              mma_f16_ss(t_dk, d_ds_k + (((kk >> 2) * kChunk + (kk & 3) * 32) >> 4), d_q_mn + kk * (2048 >> 4), idesc_dkv,
-                         (it | kk) != 0);
-            mma_commit(ds_empty);
-            mma_commit(&q_empty[n & 1]);
-            if (!next) mma_commit(fin_full);
+          };
+          if (kAlias) {          // dQ first: dP^T of the next block waits for its columns
+            if (elect_one()) {
+              issue_dq();
+              issue_dk();
+              mma_commit(ds_empty);
+              if (!next) mma_commit(fin_full);
+            }
+            __syncwarp();
+            if (next) issue_dp(n + 1, it + 2 == w.n_iter);
+          } else {               // dP^T of the next block, which the softmax warps wait for, as soon as its dO can be there
+            if (elect_one()) issue_dk();
+            __syncwarp();
+            if (next) issue_dp(n + 1, it + 2 == w.n_iter);
+            if (n > 0 && !wait(dq_empty, n - 1, MB_ERR_TIMEOUT_TMEM)) break;
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+              issue_dq();
+              mma_commit(ds_empty);
+              if (!next) mma_commit(fin_full);
+            }
+            __syncwarp();
           }
-          __syncwarp();
-          if (kAlias && next) issue_dp(n + 1, it + 2 == w.n_iter);
         }
         ++items;
       }
@@ -375,25 +431,13 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       if (t >= sch.total) break;
       const Work w = work_at(p, sch, t);
       const int kv_idx = w.kv0 + r, kv_last = w.kv0 + BB - 1;
-      auto fetch_vec = [&](int hh, int i) -> float {           // warpgroup 0 brings LSE, warpgroup 1 delta
-        const int q = (w.i_start + i) * BB + r;
-        if (part >= 2 || q >= w.sq_b) return 0.f;
-        const long at = (static_cast<long>(w.batch) * p.nh + w.unit * sch.unit_heads + hh) * p.sq + q;
-        return part ? -p.delta[at] : p.lse[at] * -1.4426950408889634f;
-      };
-      int hh = 0, i = 0;
-      if (w.n_iter > 0) {
-        const float first = fetch_vec(0, 0);
-        if (part < 2) s_vec[(n & 1) * 2 * BB + part * BB + r] = first;
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-      }
+      int i = 0;
       for (int it = 0; it < w.n_iter; ++it, ++n) {
         const int q0 = (w.i_start + i) * BB;
-        if (++i == w.per_head) { i = 0; ++hh; }
-        const float nxt = (it + 1 < w.n_iter) ? fetch_vec(hh, i) : 0.f;
+        if (++i == w.per_head) i = 0;
         const float* v_lse = s_vec + (n & 1) * 2 * BB + c0;
         const float* v_delta = v_lse + BB;
-        if (!mbar_wait(s_full, n & 1)) {
+        if (!mbar_wait(&vec_full[n & 1], (n >> 1) & 1) || !mbar_wait(s_full, n & 1)) {
           report(p.status, MB_ERR_TIMEOUT_TMEM);
           ok = false;
           break;
@@ -463,8 +507,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         fence_async_smem();
         tc_fence_before();
         mbar_arrive_warp(ds_full);
-        if (part < 2) s_vec[((n + 1) & 1) * 2 * BB + part * BB + r] = nxt;
-        asm volatile("bar.sync 1, 512;" ::: "memory");   // next block's vectors visible to all
+        mbar_arrive_warp(&vec_empty[n & 1]);
       }
       if (!ok) break;
 

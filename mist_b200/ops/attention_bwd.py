@@ -52,16 +52,19 @@ def backward(dout, q, k, v, o, lse, scale, causal, out=None, seqlens=(None, None
     elif has_native_backward():
         from .functional import Settings
         if Settings.attn_backend == "tcgen05":
-            if q.shape[2] == k.shape[2]:
-                return _native_backward(dout, q, k, v, o, lse, scale, causal, out, seqlens)
-            # grouped-query heads: every query head gets its own copy of its group's key / value head,
-            # and the gradients of the copies are summed over the group afterwards
             g = q.shape[2] // k.shape[2]
-            dq, dk, dv = _native_backward(dout, q, k.repeat_interleave(g, dim=2), v.repeat_interleave(g, dim=2),
-                                          o, lse, scale, causal, None, seqlens)
-            b, sk, nkv, d = k.shape
-            grads = (dq, dk.view(b, sk, nkv, g, d).float().sum(3).to(k.dtype),
-                     dv.view(b, sk, nkv, g, d).float().sum(3).to(v.dtype))
+            if g == 1:
+                return _native_backward(dout, q, k, v, o, lse, scale, causal, out, seqlens)
+            if not Settings.attn_bwd_pipelined:    # that kernel knows no groups: every query head gets its own copy
+                k, v = k.repeat_interleave(g, dim=2), v.repeat_interleave(g, dim=2)
+            unit = _unit_heads(q, k) if Settings.attn_bwd_pipelined else 1
+            if unit == g:
+                return _native_backward(dout, q, k, v, o, lse, scale, causal, out, seqlens, unit)
+            dq, dk, dv = _native_backward(dout, q, k, v, o, lse, scale, causal, None, seqlens, unit)
+            b, sk, n, d = dk.shape
+            parts = g // unit
+            grads = (dq, dk.view(b, sk, n // parts, parts, d).float().sum(3).to(k.dtype),
+                     dv.view(b, sk, n // parts, parts, d).float().sum(3).to(v.dtype))
         else:
             grads = _reference(dout, q, k, v, scale, causal, seqlens) if padded else _library(dout, q, k, v, scale, causal)
     else:
@@ -73,13 +76,23 @@ def backward(dout, q, k, v, o, lse, scale, causal, out=None, seqlens=(None, None
     return grads
 
 
-def _native_backward(dout, q, k, v, o, lse, scale, causal, out, seqlens=(None, None)):
+def _unit_heads(q, k) -> int:
+    """Query heads of a group that one CTA sums into dK and dV.  A CTA's longest work item is that many walks over
+    the queries; it must not exceed a CTA's share of the whole (148 CTAs, half of the blocks visible), or the last
+    CTA works alone.  What is not summed inside a CTA costs a pass over dK and dV afterwards."""
+    b, sq, nh, _ = q.shape
+    g = nh // k.shape[2]
+    most = (k.shape[1] + 127) // 128 * nh * b // 296
+    return max((u for u in range(1, g + 1) if g % u == 0 and u <= most), default=1)
+
+
+def _native_backward(dout, q, k, v, o, lse, scale, causal, out, seqlens=(None, None), unit_heads=1):
     b, sq, nh, d = q.shape
     sk = k.shape[1]
     if out is None:
         dq = torch.empty(b, sq, nh, d, dtype=q.dtype, device=q.device)
-        dk = torch.empty(b, sk, nh, d, dtype=q.dtype, device=q.device)
-        dv = torch.empty(b, sk, nh, d, dtype=q.dtype, device=q.device)
+        dk = torch.empty(b, sk, nh // unit_heads, d, dtype=q.dtype, device=q.device)
+        dv = torch.empty(b, sk, nh // unit_heads, d, dtype=q.dtype, device=q.device)
     else:
         dq, dk, dv = out
     dout = dout.contiguous()
@@ -88,7 +101,7 @@ def _native_backward(dout, q, k, v, o, lse, scale, causal, out, seqlens=(None, N
     delta = torch.empty(b, nh, sq, dtype=torch.float32, device=q.device)
     dq_acc = torch.empty(b, nh, sq, d, dtype=torch.float32, device=q.device)   # zeroed by the launch wrapper
     call("mb_attn_bwd", ptr(dout), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), ptr(delta), ptr(dq_acc),
-         ptr(dq), ptr(dk), ptr(dv), b, sq, sk, nh, d,
+         ptr(dq), ptr(dk), ptr(dv), b, sq, sk, nh, k.shape[2], unit_heads, d,
          q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
          v.stride(0), v.stride(1), v.stride(2),
          dq.stride(0), dq.stride(1), dq.stride(2), dk.stride(0), dk.stride(1), dk.stride(2),
