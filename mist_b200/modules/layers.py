@@ -459,7 +459,19 @@ class ParallelMHA(nn.Module):
             if qkv.dim() == 2:
                 qkv = qkv.view(batch_size, -1, qkv.shape[-1])
             b, s = qkv.shape[:2]
-            if self.local_heads == self.local_heads_kv:
+            # one launch over the projection's output, its gradient written the same way
+            packed = (self.use_flash_attn and not F._sym(qkv) and not self.rotary_interleaved
+                      and self.rotary_scale_base is None and (attention_mask is None or attention_mask.right_padded)
+                      and (masked or self.local_heads != self.local_heads_kv))
+            if packed:
+                rotary = None
+                if self.rotary_emb_dim > 0:        # positions are those of the padded layout
+                    rotary = (*F.rope_tables(s, self.rotary_emb_dim, self.rotary_emb_base, qkv.device),
+                              self.rotary_emb_dim)
+                ctx = F.attention_projected(qkv.view(b, s, -1, self.head_dim), self.local_heads_kv, self.softmax_scale,
+                                            self.causal, rotary,
+                                            None if attention_mask is None else attention_mask.lengths_dev)
+            elif self.local_heads == self.local_heads_kv:
                 qkv = qkv.view(b, s, 3, self.local_heads, self.head_dim)
                 rotary = None
                 # (the symbolic trace of the analyzer prices these forms like the plain rotation)
@@ -516,7 +528,12 @@ class ParallelMHA(nn.Module):
             b, sq = q.shape[:2]
             q = q.view(b, sq, self.local_heads, self.head_dim)
             kv = kv.view(b, kv.shape[1], 2, self.local_heads_kv, self.head_dim)
-            if masked:
+            if (self.use_flash_attn and not F._sym(q) and (attention_mask is None or attention_mask.right_padded)
+                    and (kv_mask is None or kv_mask.right_padded)):
+                ctx = F.attention_kvpacked(q, kv, self.softmax_scale, False,
+                                           None if attention_mask is None else attention_mask.lengths_dev,
+                                           None if kv_mask is None else kv_mask.lengths_dev)
+            elif masked:
                 ctx = self._attend_masked(q, kv[:, :, 0], kv[:, :, 1], False, attention_mask, kv_mask)
             else:
                 ctx = self._attend(q, kv[:, :, 0], kv[:, :, 1], False)

@@ -115,9 +115,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise RuntimeError(f"mb_gemm_skinny_bf16 failed with code {rc}")
     if Settings.gemm_pair and tile_n == 0:
         # returns 1 (nothing launched) when the shape or epilogue needs the single-CTA kernel
-        rc = native.kernels().mb_gemm_pair_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
-                                                out.stride(0), int(a_mn), int(b_mn), flags, ptr(bias), ptr(aux),
-                                                float(alpha), Settings.gemm_max_ctas, stream())
+        need = _pair_workspace(M, N, K, flags, Settings.gemm_max_ctas)
+        workspace = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
+        rc = native.kernels().mb_gemm_pair_split_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
+                                                      out.stride(0), int(a_mn), int(b_mn), flags, ptr(bias), ptr(aux),
+                                                      float(alpha), Settings.gemm_max_ctas, ptr(workspace), stream())
         if rc == 0:
             native.launch_count += 1
             return out
@@ -864,18 +866,20 @@ def attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k=None, scale: Optional[f
 
 
 class _PackedAttnFn(torch.autograd.Function):
-    """Rotary embedding + attention on a packed ``[b, s, 3, heads, d]`` projection output.
+    """Rotary embedding + attention on a projection output ``[b, s, q heads + 2 * kv heads, d]`` (all q heads, then
+    all k heads, then all v heads; ``[b, s, 3, heads, d]`` is that layout too).
 
     The rotation is applied in place on the projection output (nothing else keeps that
     tensor: the producing linear saves its input, not its output) and the gradient is
     produced as one packed tensor, so autograd never splits or re-concatenates q/k/v."""
 
     @staticmethod
-    def forward(ctx, qkv, cos, sin, rot, scale, causal):
+    def forward(ctx, qkv, cos, sin, rot, scale, causal, kv_heads, seqlens):
+        ctx.kv_heads, ctx.seqlens = kv_heads, seqlens
         if rot:
-            qkv = _rope_apply(qkv, cos, sin, rot, False, 2)
-        q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
-        o, lse = attn_fwd(q, k, v, scale, causal)
+            qkv = _PackedAttnFn._rotate(qkv, cos, sin, rot, False, kv_heads)
+        q, k, v = _PackedAttnFn._split(qkv, kv_heads)
+        o, lse = attn_fwd(q, k, v, scale, causal, seqlens_q=seqlens, seqlens_k=seqlens)
         ctx.rot, ctx.scale, ctx.causal = rot, scale, causal
         ctx.save_for_backward(qkv, o, lse, cos, sin)
         return o
@@ -885,16 +889,64 @@ class _PackedAttnFn(torch.autograd.Function):
         qkv, o, lse, cos, sin = ctx.saved_tensors
         from . import attention_bwd
         dqkv = torch.empty_like(qkv)
-        attention_bwd.backward(dout, qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], o, lse, ctx.scale,
-                               ctx.causal, out=(dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]))
+        attention_bwd.backward(dout, *_PackedAttnFn._split(qkv, ctx.kv_heads), o, lse, ctx.scale, ctx.causal,
+                               out=_PackedAttnFn._split(dqkv, ctx.kv_heads), seqlens=(ctx.seqlens, ctx.seqlens))
         if ctx.rot:
-            dqkv = _rope_apply(dqkv, cos, sin, ctx.rot, True, 2)
-        return dqkv, None, None, None, None, None
+            dqkv = _PackedAttnFn._rotate(dqkv, cos, sin, ctx.rot, True, ctx.kv_heads)
+        return dqkv, None, None, None, None, None, None, None
+
+
+class _KVPackedAttnFn(torch.autograd.Function):
+    """Attention of ``q`` over a projection output ``kv`` ``[b, sk, 2, kv heads, d]``, whose gradient is one tensor."""
+
+    @staticmethod
+    def forward(ctx, q, kv, scale, causal, seqlens_q, seqlens_k):
+        o, lse = attn_fwd(q, kv[:, :, 0], kv[:, :, 1], scale, causal, seqlens_q=seqlens_q, seqlens_k=seqlens_k)
+        ctx.scale, ctx.causal, ctx.seqlens = scale, causal, (seqlens_q, seqlens_k)
+        ctx.save_for_backward(q, kv, o, lse)
+        return o
+
+    @staticmethod
+    def backward(ctx, dout):
+        q, kv, o, lse = ctx.saved_tensors
+        from . import attention_bwd
+        dq, dkv = torch.empty_like(q), torch.empty_like(kv)
+        attention_bwd.backward(dout, q, kv[:, :, 0], kv[:, :, 1], o, lse, ctx.scale, ctx.causal,
+                               out=(dq, dkv[:, :, 0], dkv[:, :, 1]), seqlens=ctx.seqlens)
+        return dq, dkv, None, None, None, None
+
+
+def attention_projected(qkv, kv_heads: int, scale: float, causal: bool, rotary=None, seqlens=None):
+    """Self attention on a projection output ``[b, s, q heads + 2 * kv_heads, d]``, the gradient packed the same way.
+    ``seqlens``: as in :func:`attention`; ``rotary``: ``(cos, sin, rot_dim)``, rotated in place on the device."""
+    cos, sin, rot = rotary if rotary is not None else (None, None, 0)
+    return _PackedAttnFn.apply(qkv, cos, sin, int(rot), float(scale), bool(causal), int(kv_heads), seqlens)
+
+
+def attention_kvpacked(q, kv, scale: float, causal: bool, seqlens_q=None, seqlens_k=None):
+    """Attention of ``q`` ``[b, sq, heads, d]`` over ``kv`` ``[b, sk, 2, kv heads, d]`` with a packed ``kv`` gradient."""
+    return _KVPackedAttnFn.apply(q, kv, float(scale), bool(causal), seqlens_q, seqlens_k)
 
 
 def attention_qkvpacked(qkv, scale: Optional[float] = None, causal: bool = True, rotary=None):
     """``rotary`` is ``None`` or ``(cos, sin, rot_dim)`` from :func:`rope_tables`."""
     if _sym(qkv):
+    @staticmethod
+    def _split(qkv, nkv):
+        n = qkv.shape[2]
+        return qkv[:, :, :n - 2 * nkv], qkv[:, :, n - 2 * nkv:n - nkv], qkv[:, :, n - nkv:]
+
+    @staticmethod
+    def _rotate(qkv, cos, sin, rot, conj, nkv):
+        """q and k heads of every token; in place on the device."""
+        b, s, n, d = qkv.shape
+        if not use_native(qkv):
+            qk = _rope_apply(qkv[:, :, :n - nkv].unsqueeze(2), cos, sin, rot, conj, 1).squeeze(2)
+            return torch.cat([qk, qkv[:, :, n - nkv:]], 2)
+        assert qkv.is_contiguous()
+        call("mb_rope", ptr(qkv), ptr(cos), ptr(sin), b * s, s, n - nkv, d, rot, int(conj), 1, n * d, stream())
+        return qkv
+
         return _rules().attention_qkvpacked(qkv, scale, causal, rotary)
     if scale is None:
         scale = 1.0 / math.sqrt(qkv.shape[-1])
@@ -905,7 +957,10 @@ def attention_qkvpacked(qkv, scale: Optional[float] = None, causal: bool = True,
             qkv = _RotaryFn.apply(qkv, cos, sin, int(rot))
         q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))
         return F.scaled_dot_product_attention(q, k, v, is_causal=causal, scale=scale).transpose(1, 2)
-    return _PackedAttnFn.apply(qkv, cos, sin, int(rot), float(scale), bool(causal))
+    b, s, _, nh, d = qkv.shape
+    if rot and use_native(qkv):        # rotated in place
+        assert qkv.is_contiguous()
+    return attention_projected(qkv.reshape(b, s, 3 * nh, d), nh, scale, causal, rotary)
 
 
 class _RotaryFn(torch.autograd.Function):
