@@ -243,7 +243,9 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ ids,
     *reinterpret_cast<mb::bf16x8*>(out + t * h + c) = mb::pack8(f);
   }
 }
-// dwte[ids[t] - v0] += dout[t]   (fp32 accumulation buffer, atomics)
+// dwte[ids[t] - v0] += dout[t]   (fp32 accumulation buffer, atomics: of 16 bytes where the buffer is aligned for them,
+// since the rate is one of requests, not of bytes: 16384 tokens of 2560 values 254 -> 87 us)
+template <bool VEC>
 __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids,
                                      const __nv_bfloat16* __restrict__ dout,
                                      float* __restrict__ dwte, size_t tokens, int h, int v0,
@@ -259,8 +261,13 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids,
     float f[8];
     mb::unpack8(*reinterpret_cast<const mb::bf16x8*>(dout + t * h + c), f);
     float* dst = dwte + (id - v0) * h + c;
+    if (VEC) {
+      atomicAdd(reinterpret_cast<float4*>(dst), make_float4(f[0], f[1], f[2], f[3]));
+      atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(f[4], f[5], f[6], f[7]));
+    } else {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) atomicAdd(dst + k, f[k]);
+      for (int k = 0; k < 8; ++k) atomicAdd(dst + k, f[k]);
+    }
   }
 }
 // dwpe[s] = sum_b dout[b*seq + s]
@@ -452,8 +459,10 @@ MB_API int mb_embedding_bwd(const int64_t* ids, const void* dout, float* dwte, f
   if (h % 8) return -1;
   size_t tokens = static_cast<size_t>(batch) * seq;
   if (!tokens) return 0;
-  embedding_bwd_kernel<<<grid_for(tokens * h / 8), kBlock, 0, s>>>(ids, BF(dout), dwte, tokens, h,
-                                                                  v0, v1);
+  if ((reinterpret_cast<uintptr_t>(dwte) & 15) == 0)
+    embedding_bwd_kernel<true><<<grid_for(tokens * h / 8), kBlock, 0, s>>>(ids, BF(dout), dwte, tokens, h, v0, v1);
+  else
+    embedding_bwd_kernel<false><<<grid_for(tokens * h / 8), kBlock, 0, s>>>(ids, BF(dout), dwte, tokens, h, v0, v1);
   if (dwpe)
     pos_embedding_bwd_kernel<<<grid_for(static_cast<size_t>(seq) * h / 8), kBlock, 0, s>>>(
         BF(dout), dwpe, batch, seq, h);

@@ -149,6 +149,12 @@ class _LinearFn(torch.autograd.Function):
     def forward(ctx, x, weight, bias, activation, residual):
         ctx.activation = activation
         ctx.has_bias = bias is not None
+def _bucket_owner(weight):
+    """The parameter whose gradient bucket a backward pass writes.  What comes back from ``saved_tensors`` under saved
+    tensor hooks (a recomputed block, offloaded activations) is another tensor, without the bucket."""
+    return weight if weight.is_leaf else None
+
+
         ctx.has_residual = residual is not None
         xs = x.shape
         x2 = x.reshape(-1, xs[-1])
@@ -197,6 +203,7 @@ class _LinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         x2, weight, pre = ctx.saved_tensors
         dys = dy.shape
+        ctx.param = _bucket_owner(weight)
         dy2 = dy.reshape(-1, dys[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -218,9 +225,9 @@ class _LinearFn(torch.autograd.Function):
             dx = dx.reshape(*dys[:-1], weight.shape[1])
         dw = None
         if ctx.needs_input_grad[1]:
-            bucket = getattr(weight, "grad_bucket", None)
+            bucket = getattr(ctx.param, "grad_bucket", None)
             if bucket is not None:
-                accumulate = bool(getattr(weight, "grad_accumulate", False))
+                accumulate = bool(getattr(ctx.param, "grad_accumulate", False))
                 if tc:
                     gemm(dy2, x2, a_mn=True, b_mn=True, out=bucket,
                          flags=EPI_ACCUM if accumulate else 0)
@@ -230,7 +237,7 @@ class _LinearFn(torch.autograd.Function):
                         bucket.add_(g.to(bucket.dtype))
                     else:
                         bucket.copy_(g)
-                weight.grad_accumulate = True
+                ctx.param.grad_accumulate = True
             else:
                 if tc:
                     dw = gemm(dy2, x2, a_mn=True, b_mn=True)
@@ -272,23 +279,24 @@ class _MlpGeluFn(torch.autograd.Function):
     def backward(ctx, dy):
         x2, w1, w2, pre, act = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
+        ctx.params = _bucket_owner(w1), _bucket_owner(w2)
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
 
-        def wgrad(g, inp, weight):
-            bucket = getattr(weight, "grad_bucket", None)
+        def wgrad(g, inp, param):
+            bucket = getattr(param, "grad_bucket", None)
             if bucket is None:
                 return gemm(g, inp, a_mn=True, b_mn=True)
             gemm(g, inp, a_mn=True, b_mn=True, out=bucket,
-                 flags=EPI_ACCUM if getattr(weight, "grad_accumulate", False) else 0)
-            weight.grad_accumulate = True
+                 flags=EPI_ACCUM if getattr(param, "grad_accumulate", False) else 0)
+            param.grad_accumulate = True
             return None
 
         db2 = colsum(dy2) if (ctx.has_b2 and ctx.needs_input_grad[4]) else None
-        dw2 = wgrad(dy2, act, w2) if ctx.needs_input_grad[3] else None
+        dw2 = wgrad(dy2, act, ctx.params[1]) if ctx.needs_input_grad[3] else None
         dpre = gemm(dy2, w2, b_mn=True, aux=pre, flags=EPI_DGELU)      # (dy W2) * gelu'(pre)
         db1 = colsum(dpre) if (ctx.has_b1 and ctx.needs_input_grad[2]) else None
-        dw1 = wgrad(dpre, x2, w1) if ctx.needs_input_grad[1] else None
+        dw1 = wgrad(dpre, x2, ctx.params[0]) if ctx.needs_input_grad[1] else None
         dx = None
         if ctx.needs_input_grad[0]:
             dx = gemm(dpre, w1, b_mn=True).reshape(*dy.shape[:-1], w1.shape[1])
@@ -1104,6 +1112,7 @@ class _EmbeddingFn(torch.autograd.Function):
             inr = (loc >= 0) & (loc < wte.shape[0])
             out = wte[loc.clamp(0, wte.shape[0] - 1)].float() * inr[..., None].float()
             if wpe is not None:
+        ctx.param = _bucket_owner(wte)
                 out = out + wpe[:s].float()[None]
             return out.to(wte.dtype)
         ids = ids.contiguous()
@@ -1117,7 +1126,12 @@ class _EmbeddingFn(torch.autograd.Function):
         b, s = ids.shape
         h = wte.shape[1]
         v0, v1 = ctx.v0, ctx.v0 + wte.shape[0]
-        dwte = torch.zeros(wte.shape, dtype=torch.float32, device=wte.device)
+        bucket = getattr(ctx.param, "grad_bucket", None) if use_native(wte) and ctx.needs_input_grad[1] else None
+        accumulate = bool(getattr(ctx.param, "grad_accumulate", False))
+        if bucket is not None and bucket.dtype == torch.float32:      # summed in place
+            dwte = bucket if accumulate else bucket.zero_()
+        else:
+            dwte = torch.zeros(wte.shape, dtype=torch.float32, device=wte.device)
         dwpe = torch.zeros(wpe.shape, dtype=torch.float32, device=wte.device) if ctx.has_pos else None
         if not use_native(wte):
             loc = ids - v0
@@ -1131,7 +1145,16 @@ class _EmbeddingFn(torch.autograd.Function):
             dout = dout.contiguous()
             call("mb_embedding_bwd", ptr(ids.contiguous()), ptr(dout), ptr(dwte), ptr(dwpe), b, s, h, v0,
                  v1, stream())
-        return None, dwte.to(wte.dtype), (None if dwpe is None else dwpe.to(wpe.dtype)), None
+        dwpe = None if dwpe is None else dwpe.to(wpe.dtype)
+        if bucket is None:
+            return None, dwte.to(wte.dtype), dwpe, None
+        if dwte is not bucket:
+            if accumulate:
+                bucket.add_(dwte)
+            else:
+                cast_to_bf16(dwte, bucket)
+        ctx.param.grad_accumulate = True
+        return None, None, dwpe, None
 
 
 def embedding(ids, wte, wpe=None, vocab_start: int = 0):
