@@ -115,11 +115,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise RuntimeError(f"mb_gemm_skinny_bf16 failed with code {rc}")
     if Settings.gemm_pair and tile_n == 0:
         # returns 1 (nothing launched) when the shape or epilogue needs the single-CTA kernel
-        need = _pair_workspace(M, N, K, flags, Settings.gemm_max_ctas)
-        workspace = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
-        rc = native.kernels().mb_gemm_pair_split_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
-                                                      out.stride(0), int(a_mn), int(b_mn), flags, ptr(bias), ptr(aux),
-                                                      float(alpha), Settings.gemm_max_ctas, ptr(workspace), stream())
+        rc = native.kernels().mb_gemm_pair_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
+                                                out.stride(0), int(a_mn), int(b_mn), flags, ptr(bias), ptr(aux),
+                                                float(alpha), Settings.gemm_max_ctas, stream())
         if rc == 0:
             native.launch_count += 1
             return out
@@ -142,6 +140,12 @@ def _ref_act(x, activation):
     return x
 
 
+def _bucket_owner(weight):
+    """The parameter whose gradient bucket a backward pass writes.  What comes back from ``saved_tensors`` under saved
+    tensor hooks (a recomputed block, offloaded activations) is another tensor, without the bucket."""
+    return weight if weight.is_leaf else None
+
+
 class _LinearFn(torch.autograd.Function):
     """y = act(x W^T + b); wgrad may accumulate straight into a flat gradient bucket."""
 
@@ -149,12 +153,6 @@ class _LinearFn(torch.autograd.Function):
     def forward(ctx, x, weight, bias, activation, residual):
         ctx.activation = activation
         ctx.has_bias = bias is not None
-def _bucket_owner(weight):
-    """The parameter whose gradient bucket a backward pass writes.  What comes back from ``saved_tensors`` under saved
-    tensor hooks (a recomputed block, offloaded activations) is another tensor, without the bucket."""
-    return weight if weight.is_leaf else None
-
-
         ctx.has_residual = residual is not None
         xs = x.shape
         x2 = x.reshape(-1, xs[-1])
@@ -196,6 +194,7 @@ def _bucket_owner(weight):
                 y = fused_gather(x2)
             else:
                 y = gemm(x2, weight, bias=bias, aux=aux, flags=flags)
+        ctx.param = _bucket_owner(weight)
         ctx.save_for_backward(x2, weight, pre)
         return y.reshape(*xs[:-1], weight.shape[0])
 
@@ -203,7 +202,6 @@ def _bucket_owner(weight):
     def backward(ctx, dy):
         x2, weight, pre = ctx.saved_tensors
         dys = dy.shape
-        ctx.param = _bucket_owner(weight)
         dy2 = dy.reshape(-1, dys[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -272,6 +270,7 @@ class _MlpGeluFn(torch.autograd.Function):
         act = gemm(x2, w1, bias=b1, aux=pre, flags=EPI_GELU | EPI_SAVE_PRE)
         y = gemm(act, w2, bias=b2)
         ctx.save_for_backward(x2, w1, w2, pre, act)
+        ctx.params = _bucket_owner(w1), _bucket_owner(w2)
         ctx.has_b1, ctx.has_b2 = b1 is not None, b2 is not None
         return y.reshape(*xs[:-1], w2.shape[0])
 
@@ -279,7 +278,6 @@ class _MlpGeluFn(torch.autograd.Function):
     def backward(ctx, dy):
         x2, w1, w2, pre, act = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
-        ctx.params = _bucket_owner(w1), _bucket_owner(w2)
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
 
@@ -893,6 +891,22 @@ class _PackedAttnFn(torch.autograd.Function):
         return o
 
     @staticmethod
+    def _split(qkv, nkv):
+        n = qkv.shape[2]
+        return qkv[:, :, :n - 2 * nkv], qkv[:, :, n - 2 * nkv:n - nkv], qkv[:, :, n - nkv:]
+
+    @staticmethod
+    def _rotate(qkv, cos, sin, rot, conj, nkv):
+        """q and k heads of every token; in place on the device."""
+        b, s, n, d = qkv.shape
+        if not use_native(qkv):
+            qk = _rope_apply(qkv[:, :, :n - nkv].unsqueeze(2), cos, sin, rot, conj, 1).squeeze(2)
+            return torch.cat([qk, qkv[:, :, n - nkv:]], 2)
+        assert qkv.is_contiguous()
+        call("mb_rope", ptr(qkv), ptr(cos), ptr(sin), b * s, s, n - nkv, d, rot, int(conj), 1, n * d, stream())
+        return qkv
+
+    @staticmethod
     def backward(ctx, dout):
         qkv, o, lse, cos, sin = ctx.saved_tensors
         from . import attention_bwd
@@ -939,22 +953,6 @@ def attention_kvpacked(q, kv, scale: float, causal: bool, seqlens_q=None, seqlen
 def attention_qkvpacked(qkv, scale: Optional[float] = None, causal: bool = True, rotary=None):
     """``rotary`` is ``None`` or ``(cos, sin, rot_dim)`` from :func:`rope_tables`."""
     if _sym(qkv):
-    @staticmethod
-    def _split(qkv, nkv):
-        n = qkv.shape[2]
-        return qkv[:, :, :n - 2 * nkv], qkv[:, :, n - 2 * nkv:n - nkv], qkv[:, :, n - nkv:]
-
-    @staticmethod
-    def _rotate(qkv, cos, sin, rot, conj, nkv):
-        """q and k heads of every token; in place on the device."""
-        b, s, n, d = qkv.shape
-        if not use_native(qkv):
-            qk = _rope_apply(qkv[:, :, :n - nkv].unsqueeze(2), cos, sin, rot, conj, 1).squeeze(2)
-            return torch.cat([qk, qkv[:, :, n - nkv:]], 2)
-        assert qkv.is_contiguous()
-        call("mb_rope", ptr(qkv), ptr(cos), ptr(sin), b * s, s, n - nkv, d, rot, int(conj), 1, n * d, stream())
-        return qkv
-
         return _rules().attention_qkvpacked(qkv, scale, causal, rotary)
     if scale is None:
         scale = 1.0 / math.sqrt(qkv.shape[-1])
@@ -1105,6 +1103,7 @@ class _EmbeddingFn(torch.autograd.Function):
         h = wte.shape[1]
         ctx.v0 = v0
         ctx.has_pos = wpe is not None
+        ctx.param = _bucket_owner(wte)
         ctx.save_for_backward(ids, wte, wpe)
         v1 = v0 + wte.shape[0]
         if not use_native(wte):
@@ -1112,7 +1111,6 @@ class _EmbeddingFn(torch.autograd.Function):
             inr = (loc >= 0) & (loc < wte.shape[0])
             out = wte[loc.clamp(0, wte.shape[0] - 1)].float() * inr[..., None].float()
             if wpe is not None:
-        ctx.param = _bucket_owner(wte)
                 out = out + wpe[:s].float()[None]
             return out.to(wte.dtype)
         ids = ids.contiguous()
