@@ -42,6 +42,12 @@ struct PairParams {
   int flags;
   float alpha;
   int* status;
+  // The tiles of the last, partly filled wave (tail_tiles of them) are cut along K into `splits` parts each, so that the
+  // pairs without a tile take a share.  Every part goes to `part` in fp32; the CTA that counts the last part of its half
+  // tile in `arrived` adds them in K order and runs the epilogue.  tail_tiles = 0: nothing is split.
+  int tail_tiles, splits;
+  float* part;      // [tail tile][split][CTA of the pair][column / 4][row][4]
+  int* arrived;     // [tail tile][CTA of the pair], zero at the start
 };
 
 template <bool AUX>
@@ -90,8 +96,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
   const int num_m = (p.M + 2 * BM - 1) / (2 * BM);
   const int num_n = (p.N + BN - 1) / BN;
-  const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
+  const int full_tiles = num_m * num_n - p.tail_tiles;
+  const int num_items = full_tiles + p.tail_tiles * p.splits;
   constexpr int GM = 4;  // 256-row tiles per raster group: neighbours share B panels in L2
 
   auto tile_coords = [&](int t, int& m0, int& n0) {
@@ -102,6 +109,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     int r = t - g * per_group;
     m0 = (first_m + r % gsz) * (2 * BM) + static_cast<int>(rank) * BM;   // this CTA's rows
     n0 = (r / gsz) * BN;
+  };
+
+  // Item w of the list: tile t, K blocks [kb0, kb1); split is -1 for a whole tile.
+  auto item_at = [&](int w, int& t, int& kb0, int& kb1, int& split) {
+    t = w;
+    kb0 = 0;
+    kb1 = num_kb;
+    split = -1;
+    if (w >= full_tiles) {
+      const int u = w - full_tiles;
+      split = u / p.tail_tiles;
+      t = full_tiles + u - split * p.tail_tiles;
+      kb0 = split * num_kb / p.splits;
+      kb1 = (split + 1) * num_kb / p.splits;
+    }
   };
 
   if (threadIdx.x == 0) {
@@ -135,11 +157,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       uint32_t armed[STAGES];
       for (int s = 0; s < STAGES; ++s) armed[s] = 0;
       bool ok = true;
-      for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        int m0, n0;
+      for (int w = pair; w < num_items && ok; w += num_pairs) {
+        int t, kb0, kb1, split, m0, n0;
+        item_at(w, t, kb0, kb1, split);
         tile_coords(t, m0, n0);
         const int nb0 = n0 + static_cast<int>(rank) * BNH;   // this CTA's rows of B
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           int s = it % STAGES;
           uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
@@ -180,7 +203,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       uint32_t it = 0, tcount = 0;
       bool ok = true;
-      for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tcount) {
+      for (int w = pair; w < num_items && ok; w += num_pairs, ++tcount) {
+        int t, kb0, kb1, split;
+        item_at(w, t, kb0, kb1, split);
         int acc = tcount & 1;
         uint32_t acc_ph = (tcount >> 1) & 1;
         if (!mbar_wait(&tempty_bar[acc], acc_ph ^ 1)) {
@@ -190,7 +215,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
         tc_fence_after();
         uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           int s = it % STAGES;
           uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&full_bar[s], ph)) {
@@ -208,7 +233,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                                  : make_smem_desc_sw128(sa + k * 32, 16, 1024);
               uint64_t bd = B_MN ? make_smem_desc_sw128(sb + k * 2048, BK * 128, 1024)
                                  : make_smem_desc_sw128(sb + k * 32, 16, 1024);
-              mma_f16_ss_pair(d_tmem, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
+              mma_f16_ss_pair(d_tmem, ad, bd, idesc, ((kb - kb0) | k) != 0 ? 1u : 0u);
             }
             mma_commit_pair(&empty_bar[s]);   // frees the stage in both CTAs
           }
@@ -229,8 +254,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const int npass = (p.flags & EPI_SAVE_PRE) ? 2 : 1;
     uint32_t tcount = 0, epi_units = 0, aux_units = 0;
     bool ok = true;
-    for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tcount) {
-      int m0, n0;
+    for (int w = pair; w < num_items && ok; w += num_pairs, ++tcount) {
+      int t, kb0, kb1, split, m0, n0;
+      item_at(w, t, kb0, kb1, split);
       tile_coords(t, m0, n0);
       int acc = tcount & 1;
       uint32_t acc_ph = (tcount >> 1) & 1;
@@ -251,6 +277,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
+      auto release_accumulator = [&]() {     // tell the leader's MMA warp (one arrival per warp)
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+      };
+      const float4* parts = nullptr;         // the tile's parts in K order, where it was split
+      if (!AUX && split >= 0) {
+        constexpr int kPart4 = BM * BN / 4;  // float4s of a CTA's half of a part
+        const int tail = t - full_tiles;
+        float4* all = reinterpret_cast<float4*>(p.part) + static_cast<size_t>(tail) * p.splits * 2 * kPart4 + rank * kPart4 + r;
+        float4* mine = all + static_cast<size_t>(split) * 2 * kPart4;
+        for (int c = 0; c < BN; c += 32) {
+          uint32_t rr[32];
+          tmem_ld32(taddr + c, rr);
+          tmem_ld_wait();
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            mine[(c / 4 + g) * BM] = make_float4(__uint_as_float(rr[4 * g]), __uint_as_float(rr[4 * g + 1]),
+                                                 __uint_as_float(rr[4 * g + 2]), __uint_as_float(rr[4 * g + 3]));
+        }
+        release_accumulator();
+        __threadfence();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (leader) tmem_slot[1] = (atomicAdd(&p.arrived[2 * tail + rank], 1) == p.splits - 1);
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (!tmem_slot[1]) continue;
+        __threadfence();
+        parts = all;
+      }
       const bool rows_live = m0 < p.M;   // the second CTA of a pair can hang over the bottom edge
       int units_live = 0;
       if (rows_live) units_live = min(units, (p.N - n0 + cols_per_unit - 1) / cols_per_unit);
@@ -271,13 +326,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           asm volatile("bar.sync 1, 128;" ::: "memory");
           const int halves = out_fp32 ? 1 : 2;
           for (int hh = 0; hh < halves; ++hh) {
-            uint32_t rr[32];
-            tmem_ld32(taddr + u * cols_per_unit + hh * 32, rr);
-            tmem_ld_wait();
             float v[32];
             const int col0 = ucol0 + hh * 32;
+            if (!AUX && parts) {
+              const float4* at = parts + (u * cols_per_unit + hh * 32) / 4 * BM;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(rr[i]) * p.alpha;
+              for (int i = 0; i < 32; ++i) v[i] = 0.f;
+              for (int sp = 0; sp < p.splits; ++sp, at += 2 * (BM * BN / 4)) {
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                  const float4 x = __ldcg(at + g * BM);
+                  v[4 * g] += x.x; v[4 * g + 1] += x.y; v[4 * g + 2] += x.z; v[4 * g + 3] += x.w;
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] *= p.alpha;
+            } else {
+              uint32_t rr[32];
+              tmem_ld32(taddr + u * cols_per_unit + hh * 32, rr);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(rr[i]) * p.alpha;
+            }
             if (p.flags & EPI_BIAS) {
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] += __bfloat162float(p.bias[min(col0 + i, p.N - 1)]);
@@ -337,10 +407,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
       }
       aux_units += units_live;
-      // accumulator stage read: tell the leader's MMA warp (one arrival per warp)
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+      if (AUX || split < 0) release_accumulator();
     }
     if (leader) tma_wait_all<0>();
   }
@@ -388,6 +455,40 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
 }
 
 int g_sms = 0;
+
+struct Split {
+  int tail_tiles, splits;
+};
+// How the last wave is cut.  A part costs its share of the K blocks, and 4 K blocks (of about 0.3 us) for each part that
+// is written and read back; a split has to save 8 K blocks.  So it is the long sums with a nearly empty last wave that
+// are split, above all weight gradients, whose K is the number of tokens: 16384 tokens, 7680 x 2560 (300 tiles on 74 pairs)
+// 490 -> 446 us; 8192 tokens, 4096 x 4096 (256 tiles) 208 -> 193 us, 4096 x 11008 (688 tiles) 700 -> 644 us.
+Split choose_split(int M, int N, int K, int flags, int max_ctas) {
+  Split none = {0, 1};
+  const int pairs = max_ctas / 2, num_kb = (K + BK - 1) / BK;
+  const long tiles = static_cast<long>((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+  if (pairs < 1 || tiles < pairs || (flags & (EPI_DGELU | EPI_RESIDUAL))) return none;
+  const int tail = static_cast<int>(tiles % pairs);
+  int best = num_kb - 8, splits = 1;
+  for (int s = 2; s <= 8 && tail > 0 && num_kb / s >= 8; ++s) {
+    const int cost = (s * tail + pairs - 1) / pairs * ((num_kb + s - 1) / s) + 4 * (s + 1);
+    if (cost <= best) {
+      best = cost - 1;
+      splits = s;
+    }
+  }
+  if (splits == 1) return none;
+  return {tail, splits};
+}
+int clamp_ctas(int max_ctas) {
+  if (!g_sms) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return (max_ctas <= 0 || max_ctas > g_sms) ? g_sms : max_ctas;
+}
+size_t arrived_bytes(const Split& s) { return (static_cast<size_t>(s.tail_tiles) * 2 * 4 + 255) / 256 * 256; }
 
 template <bool A_MN, bool B_MN, bool AUX>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx,
@@ -441,9 +542,19 @@ static char g_pair_err[256] = "";
 // Arguments of the last mb_gemm_pair_bf16 call that got as far as building its tensor maps.
 MB_API const char* mb_gemm_pair_last_error(void) { return g_pair_err; }
 
-MB_API int mb_gemm_pair_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                             int a_mn_major, int b_mn_major, int flags, const void* bias, void* aux, float alpha,
-                             int max_ctas, cudaStream_t stream) {
+// Bytes of workspace with which mb_gemm_pair_bf16 would split the tiles of its last wave; 0: nothing to split.
+MB_API size_t mb_gemm_pair_workspace(int M, int N, int K, int flags, int max_ctas) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const Split s = choose_split(M, N, K, flags, clamp_ctas(max_ctas));
+  if (!s.tail_tiles) return 0;
+  return arrived_bytes(s) + static_cast<size_t>(s.tail_tiles) * s.splits * 2 * BM * BN * sizeof(float);
+}
+
+// mb_gemm_pair_bf16 (below) with a workspace of as many bytes as mb_gemm_pair_workspace says, aligned to 16 and for this
+// call alone; null: no tile is split.
+MB_API int mb_gemm_pair_split_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
+                                   int ldc, int a_mn_major, int b_mn_major, int flags, const void* bias, void* aux,
+                                   float alpha, int max_ctas, void* workspace, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
     return -1;
@@ -461,12 +572,7 @@ MB_API int mb_gemm_pair_bf16(const void* A, const void* B, void* C, int M, int N
         ((flags & EPI_DGELU) && (flags & EPI_RESIDUAL)))
       return 1;
   }
-  if (!g_sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  if (max_ctas <= 0 || max_ctas > g_sms) max_ctas = g_sms;
+  max_ctas = clamp_ctas(max_ctas);
   const long tiles = static_cast<long>((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
   if (tiles < max_ctas / 2) return 1;     // cannot fill the machine with 256 x 256 tiles
   CUtensorMap ta, tb, tc, tx;
@@ -490,6 +596,20 @@ MB_API int mb_gemm_pair_bf16(const void* A, const void* B, void* C, int M, int N
   p.flags = flags;
   p.alpha = alpha;
   p.status = mb_status_device_ptr();
+  Split split = {0, 1};
+  if (workspace && !(reinterpret_cast<uintptr_t>(workspace) & 15)) split = choose_split(M, N, K, flags, max_ctas);
+  p.tail_tiles = split.tail_tiles;
+  p.splits = split.splits;
+  p.arrived = reinterpret_cast<int*>(workspace);
+  p.part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + arrived_bytes(split));
+  if (split.tail_tiles && cudaMemsetAsync(workspace, 0, arrived_bytes(split), stream) != cudaSuccess) return -4;
   if (has_aux) return dispatch<true>(a_mn_major != 0, b_mn_major != 0, ta, tb, tc, tx, p, max_ctas, stream);
   return dispatch<false>(a_mn_major != 0, b_mn_major != 0, ta, tb, tc, tx, p, max_ctas, stream);
+}
+
+MB_API int mb_gemm_pair_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                             int a_mn_major, int b_mn_major, int flags, const void* bias, void* aux, float alpha,
+                             int max_ctas, cudaStream_t stream) {
+  return mb_gemm_pair_split_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, flags, bias, aux, alpha,
+                                 max_ctas, nullptr, stream);
 }

@@ -15,6 +15,7 @@ The ops mirror the fused operators the reference's module library is built on
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from typing import Optional
@@ -84,6 +85,12 @@ def _get_scratch(numel: int, device, key="default") -> torch.Tensor:
 
 
 # ------------------------------------------------------------------------------ GEMM
+@functools.lru_cache(maxsize=4096)
+def _pair_workspace(M: int, N: int, K: int, flags: int, max_ctas: int) -> int:
+    """Bytes that the CTA-pair GEMM wants for the split tiles of its last wave; a function of the sizes alone."""
+    return native.kernels().mb_gemm_pair_workspace(M, N, K, flags, max_ctas)
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype=torch.bfloat16, bias=None, aux=None,
          flags: int = 0, alpha: float = 1.0, tile_n: int = 0) -> torch.Tensor:
@@ -115,9 +122,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise RuntimeError(f"mb_gemm_skinny_bf16 failed with code {rc}")
     if Settings.gemm_pair and tile_n == 0:
         # returns 1 (nothing launched) when the shape or epilogue needs the single-CTA kernel
-        rc = native.kernels().mb_gemm_pair_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
-                                                out.stride(0), int(a_mn), int(b_mn), flags, ptr(bias), ptr(aux),
-                                                float(alpha), Settings.gemm_max_ctas, stream())
+        need = _pair_workspace(M, N, K, flags, Settings.gemm_max_ctas)
+        workspace = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
+        rc = native.kernels().mb_gemm_pair_split_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
+                                                      out.stride(0), int(a_mn), int(b_mn), flags, ptr(bias), ptr(aux),
+                                                      float(alpha), Settings.gemm_max_ctas, ptr(workspace), stream())
         if rc == 0:
             native.launch_count += 1
             return out

@@ -33,6 +33,8 @@ _SIGNATURES = {
     "mb_status_read_and_clear": ([], _i),
     "mb_status_device_ptr": ([], _p),
     "mb_gemm_bf16": ([_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p, _p, _f, _i, _i, _p], _i),
+    "mb_gemm_pair_split_bf16": ([_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p, _p, _f, _i, _p, _p], _i),
+    "mb_gemm_pair_workspace": ([_i, _i, _i, _i, _i], _z),
     "mb_gemm_pair_bf16": ([_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p, _p, _f, _i, _p], _i),
     "mb_decode_attn": ([_p, _p, _p, _p, _i, _i, _i, _i, _i, _l, _l, _l, _l, _l, _l, _l, _f, _i, _p], _i),
     "mb_rope_append": ([_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _l, _i, _p], _i),
