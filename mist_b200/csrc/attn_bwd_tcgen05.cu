@@ -462,6 +462,30 @@ __global__ void attn_convert_dq_kernel(const float* __restrict__ acc, __nv_bfloa
   }
 }
 
+// dk[b][t][h][:] = sum of the `parts` consecutive heads of dk_parts that belong to h, dv likewise (blockIdx.y); fp32 sums.
+__global__ void __launch_bounds__(256)
+attn_sum_parts_kernel(const __nv_bfloat16* __restrict__ dk_parts, const __nv_bfloat16* __restrict__ dv_parts,
+                      __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long total, int sk, int nh_kv,
+                      int parts, int d, long dk_bs, long dk_ts, long dk_hs, long dv_bs, long dv_ts, long dv_hs) {
+  const long i = blockIdx.x * 256l + threadIdx.x;
+  if (i >= total) return;
+  const int vpr = d >> 3;
+  const long row = i / vpr;                      // (b, t, h)
+  const int v = static_cast<int>(i - row * vpr), h = static_cast<int>(row % nh_kv);
+  const long bt = row / nh_kv, b = bt / sk, t = bt - b * sk;
+  const bool is_v = blockIdx.y != 0;
+  const __nv_bfloat16* src = (is_v ? dv_parts : dk_parts) + row * parts * d + 8 * v;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int p = 0; p < parts; ++p) {
+    float f[8];
+    mb::unpack8(*reinterpret_cast<const mb::bf16x8*>(src + p * d), f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[k] += f[k];
+  }
+  __nv_bfloat16* dst = is_v ? dv + b * dv_bs + t * dv_ts + h * dv_hs : dk + b * dk_bs + t * dk_ts + h * dk_hs;
+  *reinterpret_cast<mb::bf16x8*>(dst + 8 * v) = mb::pack8(acc);
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -617,5 +641,23 @@ MB_API int mb_attn_bwd(const void* dout, const void* q, const void* k, const voi
     attn_convert_dq_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
         dq_acc, reinterpret_cast<__nv_bfloat16*>(dq), batch, sq, nh, d, dq_bs, dq_ts, dq_hs, pipelined ? scale : 1.f);
   }
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+// dk_parts, dv_parts: contiguous [b][sk][nh_kv * parts][d]; dk, dv: [b][sk][nh_kv][d] with the given element strides
+// (multiples of 8).
+MB_API int mb_attn_sum_parts(const void* dk_parts, const void* dv_parts, void* dk, void* dv, int batch, int sk, int nh_kv,
+                             int parts, int d, long dk_bs, long dk_ts, long dk_hs, long dv_bs, long dv_ts, long dv_hs,
+                             cudaStream_t stream) {
+  if (d % 8 || ((dk_bs | dk_ts | dk_hs | dv_bs | dv_ts | dv_hs) & 7) || parts < 1) return -1;
+  if ((reinterpret_cast<uintptr_t>(dk_parts) | reinterpret_cast<uintptr_t>(dv_parts) | reinterpret_cast<uintptr_t>(dk) |
+       reinterpret_cast<uintptr_t>(dv)) & 15)
+    return -1;
+  const long total = static_cast<long>(batch) * sk * nh_kv * (d / 8);
+  if (!total) return 0;
+  attn_sum_parts_kernel<<<dim3(static_cast<unsigned>((total + 255) / 256), 2), 256, 0, stream>>>(
+      reinterpret_cast<const __nv_bfloat16*>(dk_parts), reinterpret_cast<const __nv_bfloat16*>(dv_parts),
+      reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(dv), total, sk, nh_kv, parts, d, dk_bs, dk_ts,
+      dk_hs, dv_bs, dv_ts, dv_hs);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

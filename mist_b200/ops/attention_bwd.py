@@ -60,11 +60,16 @@ def backward(dout, q, k, v, o, lse, scale, causal, out=None, seqlens=(None, None
             unit = _unit_heads(q, k) if Settings.attn_bwd_pipelined else 1
             if unit == g:
                 return _native_backward(dout, q, k, v, o, lse, scale, causal, out, seqlens, unit)
-            dq, dk, dv = _native_backward(dout, q, k, v, o, lse, scale, causal, None, seqlens, unit)
-            b, sk, n, d = dk.shape
-            parts = g // unit
-            grads = (dq, dk.view(b, sk, n // parts, parts, d).float().sum(3).to(k.dtype),
-                     dv.view(b, sk, n // parts, parts, d).float().sum(3).to(v.dtype))
+            b, sk, nkv, d = k.shape if Settings.attn_bwd_pipelined else (*k.shape[:2], k.shape[2] // g, k.shape[3])
+            if out is None:
+                out = (torch.empty_like(q, memory_format=torch.contiguous_format),
+                       *(torch.empty(b, sk, nkv, d, dtype=q.dtype, device=q.device) for _ in range(2)))
+            dq, dk, dv = out
+            part_k, part_v = (torch.empty(b, sk, nkv * (g // unit), d, dtype=q.dtype, device=q.device) for _ in range(2))
+            _native_backward(dout, q, k, v, o, lse, scale, causal, (dq, part_k, part_v), seqlens, unit)
+            call("mb_attn_sum_parts", ptr(part_k), ptr(part_v), ptr(dk), ptr(dv), b, sk, nkv, g // unit, d,
+                 dk.stride(0), dk.stride(1), dk.stride(2), dv.stride(0), dv.stride(1), dv.stride(2), stream())
+            return out
         else:
             grads = _reference(dout, q, k, v, scale, causal, seqlens) if padded else _library(dout, q, k, v, scale, causal)
     else:

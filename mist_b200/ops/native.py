@@ -68,6 +68,7 @@ _SIGNATURES = {
     "mb_causal_softmax_bwd": ([_p, _p, _p, _z, _i, _f, _p], _i),
     "mb_adam_step": ([_p, _p, _p, _p, _i, _p, _z, _f, _f, _f, _f, _f, _i, _f, _i, _p], _i),
     "mb_attn_bwd": ([_p] * 11 + [_i] * 7 + [_l] * 18 + [_f, _i, _p, _p, _p], _i),
+    "mb_attn_sum_parts": ([_p] * 4 + [_i] * 5 + [_l] * 6 + [_p], _i),
     "mb_attn_fwd": ([_p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i] + [_l] * 12 + [_f, _i, _p, _p, _p], _i),
 }
 

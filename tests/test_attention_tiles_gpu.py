@@ -91,3 +91,21 @@ def test_block_kernels_on_padded_batches(d, causal):
     native.check_status()
     for got, want in zip(grads, torch.autograd.grad(o_ref, leaves, g.double())):
         _close(got, want)
+
+
+@pytest.mark.parametrize("nh,nkv,s", [(8, 2, 300), (4, 4, 257), (16, 4, 2048)])
+def test_gradients_into_a_packed_projection(nh, nkv, s):
+    """dK and dV of a group, summed over parts or in the CTA, land in strided views of one gradient."""
+    torch.manual_seed(s)
+    b, d, scale = 2, 80, 0.11
+    qkv = torch.randn(b, s, nh + 2 * nkv, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    g = torch.randn(b, s, nh, d, device=DEV, dtype=torch.bfloat16)
+    o = F.attention_projected(qkv, nkv, scale, True)
+    o.backward(g)
+    native.check_status()
+    leaf = qkv.detach().double().requires_grad_(True)
+    o_ref, _ = _exact(*leaf.split([nh, nkv, nkv], 2), scale, True)
+    o_ref.backward(g.double())
+    _close(o, o_ref)
+    for got, want in zip(qkv.grad.split([nh, nkv, nkv], 2), leaf.grad.split([nh, nkv, nkv], 2)):
+        _close(got, want)
