@@ -323,6 +323,23 @@ __global__ void colsum_stage2(const float* __restrict__ part, OutT* __restrict__
 }
 
 // ------------------------------------------------------------------- casts
+// dst = bf16(dst + src): the sum is rounded once
+__global__ void add_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, size_t n) {
+  const size_t nvec = n >> 3;
+  for (size_t i = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x; i < nvec;
+       i += static_cast<size_t>(gridDim.x) * kBlock) {
+    const float4 a = reinterpret_cast<const float4*>(src)[2 * i], b = reinterpret_cast<const float4*>(src)[2 * i + 1];
+    float f[8];
+    mb::unpack8(reinterpret_cast<const mb::bf16x8*>(dst)[i], f);
+    f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+    f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+    reinterpret_cast<mb::bf16x8*>(dst)[i] = mb::pack8(f);
+  }
+  if (blockIdx.x == 0 && threadIdx.x < (n & 7)) {
+    const size_t j = (nvec << 3) + threadIdx.x;
+    dst[j] = __float2bfloat16(__bfloat162float(dst[j]) + src[j]);
+  }
+}
 __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out,
                                         size_t n, float scale) {
   const size_t nvec = n >> 3;
@@ -488,6 +505,11 @@ MB_API int mb_colsum(const void* x, void* out, float* scratch, int rows, int col
 MB_API int mb_cast_f32_to_bf16(const float* in, void* out, size_t n, float scale, cudaStream_t s) {
   if (!n) return 0;
   cast_f32_to_bf16_kernel<<<grid_for((n + 7) / 8), kBlock, 0, s>>>(in, BFM(out), n, scale);
+  return LAUNCH_OK();
+}
+MB_API int mb_add_f32_to_bf16(const float* src, void* dst, size_t n, cudaStream_t s) {
+  if (!n) return 0;
+  add_f32_to_bf16_kernel<<<grid_for((n + 7) / 8), kBlock, 0, s>>>(src, BFM(dst), n);
   return LAUNCH_OK();
 }
 MB_API int mb_axpy_bf16_to_f32(const void* src, float* dst, size_t n, float scale, int accumulate,

@@ -1157,7 +1157,7 @@ class _EmbeddingFn(torch.autograd.Function):
             return None, dwte.to(wte.dtype), dwpe, None
         if dwte is not bucket:
             if accumulate:
-                bucket.add_(dwte)
+                call("mb_add_f32_to_bf16", ptr(dwte), ptr(bucket), dwte.numel(), stream())
             else:
                 cast_to_bf16(dwte, bucket)
         ctx.param.grad_accumulate = True

@@ -60,6 +60,7 @@ _SIGNATURES = {
     "mb_colsum": ([_p, _p, _p, _i, _i, _i, _i, _p], _i),
     "mb_cast_f32_to_bf16": ([_p, _p, _z, _f, _p], _i),
     "mb_axpy_bf16_to_f32": ([_p, _p, _z, _f, _i, _p], _i),
+    "mb_add_f32_to_bf16": ([_p, _p, _z, _p], _i),
     "mb_add_bf16": ([_p, _p, _z, _p], _i),
     "mb_xent_stats": ([_p, _p, _p, _i, _i, _i, _i, _p], _i),
     "mb_xent_loss": ([_p, _p, _p, _p, _i, _i, _p], _i),

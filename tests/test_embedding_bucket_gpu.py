@@ -1,0 +1,34 @@
+"""Embedding gradients summed into the flat bucket, against an fp32 scatter.
+
+The fp32 sums differ by the order of the atomics (2^-22 of values of a few units here); a bf16 bucket is rounded once."""
+import pytest
+import torch
+
+from mist_b200.ops import functional as F
+from mist_b200.ops import native
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("offset", [0, 2])          # elements before the bucket: 16-byte atomics need aligned rows
+def test_embedding_bucket(dtype, accumulate, offset):
+    if dtype == torch.bfloat16 and offset:
+        pytest.skip("bf16 buckets start on 16 bytes")
+    torch.manual_seed(1)
+    v, h, start = 37, 24, 5
+    w = torch.nn.Parameter(torch.randn(v, h, device=DEV, dtype=torch.bfloat16))
+    ids = torch.randint(0, v + 2 * start, (3, 50), device=DEV)          # some outside this rank's slice
+    g = torch.randn(3, 50, h, device=DEV, dtype=torch.bfloat16)
+    bucket = torch.randn(offset + v * h, device=DEV).to(dtype)[offset:].view(v, h)
+    old = bucket.float().clone() if accumulate else torch.zeros(v, h, device=DEV)
+    w.grad_bucket, w.grad_accumulate = bucket, accumulate
+    F.embedding(ids, w, None, start).backward(g)
+    native.check_status()
+    inside = ((ids >= start) & (ids < start + v)).reshape(-1)
+    want = old.double().index_add(0, (ids.reshape(-1) - start)[inside], g.double().reshape(-1, h)[inside])
+    assert w.grad is None and w.grad_accumulate
+    bound = 2 ** -20 if dtype == torch.float32 else 2 ** -8
+    assert ((bucket.double() - want).abs() <= bound * want.abs().clamp(min=1.0)).all()
