@@ -416,29 +416,42 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
 #include "attn_bwd_wide_tcgen05.cuh"
 
-// delta[b][h][q] = sum_d dO[b][q][h][d] * O[b][q][h][d]; sixteen lanes per (b, q, h), one vector each
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o,
-                                  float* __restrict__ delta, int batch, int sq, int nh, int d, long do_bs,
-                                  long do_ts, long do_hs, long o_bs, long o_ts, long o_hs) {
-  const long w = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
+// delta[b][h][q] = sum_d dO[b][q][h][d] * O[b][q][h][d]; sixteen lanes per (b, q, h), one vector each, and four rows at a
+// time so that eight loads of a thread are in flight.
+constexpr int kDeltaRows = 4;
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o,
+                  float* __restrict__ delta, int batch, int sq, int nh, int d, long do_bs,
+                  long do_ts, long do_hs, long o_bs, long o_ts, long o_hs) {
+  const unsigned first = ((blockIdx.x * 256u + threadIdx.x) >> 4) * kDeltaRows;
   const int sub = threadIdx.x & 15;
-  const long total = static_cast<long>(batch) * sq * nh;
-  const long row = w < total ? w : total - 1;      // the last warp stays whole for the shuffles
-  const int h = static_cast<int>(row % nh);
-  const long t = row / nh;
-  const int q = static_cast<int>(t % sq);
-  const int b = static_cast<int>(t / sq);
-  float acc = 0.f;
-  if (sub * 8 < d) {
-    float x[8], y[8];
-    mb::unpack8(*reinterpret_cast<const mb::bf16x8*>(dout + b * do_bs + q * do_ts + h * do_hs + sub * 8), x);
-    mb::unpack8(*reinterpret_cast<const mb::bf16x8*>(o + b * o_bs + q * o_ts + h * o_hs + sub * 8), y);
+  const unsigned total = static_cast<unsigned>(batch) * sq * nh;
+  mb::bf16x8 x[kDeltaRows], y[kDeltaRows];
+  unsigned at[kDeltaRows];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc += x[k] * y[k];
+  for (int u = 0; u < kDeltaRows; ++u) {
+    const unsigned row = min(first + u, total - 1);      // the last warp stays whole for the shuffles
+    const unsigned t = row / nh, h = row - t * nh, b = t / sq, q = t - b * sq;
+    at[u] = (b * nh + h) * sq + q;
+    if (sub * 8 < d) {
+      x[u] = *reinterpret_cast<const mb::bf16x8*>(dout + b * do_bs + q * do_ts + h * do_hs + sub * 8);
+      y[u] = *reinterpret_cast<const mb::bf16x8*>(o + b * o_bs + q * o_ts + h * o_hs + sub * 8);
+    }
   }
 #pragma unroll
-  for (int m = 8; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-  if (sub == 0 && w < total) delta[(static_cast<long>(b) * nh + h) * sq + q] = acc;
+  for (int u = 0; u < kDeltaRows; ++u) {
+    float acc = 0.f;
+    if (sub * 8 < d) {
+      float f[8], g[8];
+      mb::unpack8(x[u], f);
+      mb::unpack8(y[u], g);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc += f[k] * g[k];
+    }
+#pragma unroll
+    for (int m = 8; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    if (sub == 0 && first + u < total) delta[at[u]] = acc;
+  }
 }
 
 // dq[b][q][h][:] = bf16(scale * dq_acc[b][h][q][:])
@@ -571,7 +584,8 @@ MB_API int mb_attn_bwd(const void* dout, const void* q, const void* k, const voi
   const long o_ts = static_cast<long>(nh) * d, o_bs = o_ts * sq;
   {
     long rows = static_cast<long>(batch) * sq * nh;
-    long blocks = (rows * 16 + 255) / 256;
+    if (rows > 0x7fffffff) return -1;
+    long blocks = (rows + 16 * kDeltaRows - 1) / (16 * kDeltaRows);
     attn_delta_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
         reinterpret_cast<const __nv_bfloat16*>(dout), reinterpret_cast<const __nv_bfloat16*>(o), delta, batch, sq,
         nh, d, o_bs, o_ts, d, o_bs, o_ts, d);
