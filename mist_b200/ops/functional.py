@@ -890,7 +890,9 @@ class _PackedAttnFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, cos, sin, rot, scale, causal, kv_heads, seqlens):
-        ctx.kv_heads, ctx.seqlens = kv_heads, seqlens
+        ctx.kv_heads, ctx.seqlens, ctx.shape = kv_heads, seqlens, qkv.shape
+        if qkv.dim() == 5:
+            qkv = qkv.reshape(*qkv.shape[:2], -1, qkv.shape[4])
         if rot:
             qkv = _PackedAttnFn._rotate(qkv, cos, sin, rot, False, kv_heads)
         q, k, v = _PackedAttnFn._split(qkv, kv_heads)
@@ -924,7 +926,7 @@ class _PackedAttnFn(torch.autograd.Function):
                                out=_PackedAttnFn._split(dqkv, ctx.kv_heads), seqlens=(ctx.seqlens, ctx.seqlens))
         if ctx.rot:
             dqkv = _PackedAttnFn._rotate(dqkv, cos, sin, ctx.rot, True, ctx.kv_heads)
-        return dqkv, None, None, None, None, None, None, None
+        return dqkv.view(ctx.shape), None, None, None, None, None, None, None
 
 
 class _KVPackedAttnFn(torch.autograd.Function):
@@ -948,7 +950,8 @@ class _KVPackedAttnFn(torch.autograd.Function):
 
 
 def attention_projected(qkv, kv_heads: int, scale: float, causal: bool, rotary=None, seqlens=None):
-    """Self attention on a projection output ``[b, s, q heads + 2 * kv_heads, d]``, the gradient packed the same way.
+    """Self attention on a projection output ``[b, s, q heads + 2 * kv_heads, d]`` or ``[b, s, 3, kv_heads, d]``, the
+    gradient packed the same way.
     ``seqlens``: as in :func:`attention`; ``rotary``: ``(cos, sin, rot_dim)``, rotated in place on the device."""
     cos, sin, rot = rotary if rotary is not None else (None, None, 0)
     return _PackedAttnFn.apply(qkv, cos, sin, int(rot), float(scale), bool(causal), int(kv_heads), seqlens)
@@ -972,10 +975,9 @@ def attention_qkvpacked(qkv, scale: Optional[float] = None, causal: bool = True,
             qkv = _RotaryFn.apply(qkv, cos, sin, int(rot))
         q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))
         return F.scaled_dot_product_attention(q, k, v, is_causal=causal, scale=scale).transpose(1, 2)
-    b, s, _, nh, d = qkv.shape
     if rot and use_native(qkv):        # rotated in place
         assert qkv.is_contiguous()
-    return attention_projected(qkv.reshape(b, s, 3 * nh, d), nh, scale, causal, rotary)
+    return attention_projected(qkv, qkv.shape[3], scale, causal, rotary)
 
 
 class _RotaryFn(torch.autograd.Function):

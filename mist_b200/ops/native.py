@@ -137,7 +137,9 @@ def use_native(*tensors) -> bool:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle of the current stream: a Stream object for each of a step's launches costs the host more than the
+    # launch arguments do
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t) -> int:
