@@ -431,7 +431,7 @@ class ParallelMHA(nn.Module):
         else:
             qk = qkv[..., : (hq + hk) * d].reshape(b, s, 1, hq + hk, d)
             if rotary is not None:
-                qk = F._rope_apply(qk.contiguous().clone(), *rotary, False, 1)
+                qk = _RotaryOutOfPlace.apply(qk, *rotary, 1)
             qk = qk.reshape(b, s, hq + hk, d)
             q, k = qk[:, :, :hq], qk[:, :, hq:]
             v = qkv[..., (hq + hk) * d:].reshape(b, s, hk, d)

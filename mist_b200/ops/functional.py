@@ -754,8 +754,10 @@ def decode_attention(q, k_cache, v_cache, seq_len: int, scale: Optional[float] =
 
 
 def rope_append_available(qkv, cache, rot: int, d: int) -> bool:
-    return (not _sym(qkv) and use_native(qkv) and qkv.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16
-            and d % 8 == 0 and rot % 16 == 0)
+    """Whether :func:`rope_append_` may take ``qkv``; it works outside autograd, so not where a gradient is recorded."""
+    recorded = torch.is_grad_enabled() and (qkv.requires_grad or cache.requires_grad)
+    return (not _sym(qkv) and not recorded and use_native(qkv) and qkv.dtype == torch.bfloat16
+            and cache.dtype == torch.bfloat16 and d % 8 == 0 and rot % 16 == 0)
 
 
 def rope_append_(qkv, cache, offset: int, hq: int, hk: int, d: int, rotary=None):
