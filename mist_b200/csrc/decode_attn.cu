@@ -400,6 +400,7 @@ MB_API int mb_decode_attn(const void* q, const void* k, const void* v, void* o, 
   if (batch <= 0 || nh <= 0) return 0;
   if (d % 8 || d > kMaxD || d <= 0 || nh_kv <= 0 || nh % nh_kv || len < 1) return -1;
   if ((q_sb | k_sb | k_ss | k_sh | v_sb | v_ss | v_sh) & 7) return -1;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) return -1;
   const int group = nh / nh_kv;
   const float sl = scale * 1.4426950408889634f;
 #define MB_DECODE(L_, G_, S_)                                                                                        \
@@ -420,10 +421,11 @@ MB_API int mb_decode_attn(const void* q, const void* k, const void* v, void* o, 
 #undef MB_DECODE
 }
 
-// See rope_append_kernel.  rot % 16 == 0 (0: no rotation, cos / sin unused), d % 8 == 0.
+// See rope_append_kernel.  rot % 16 == 0 (0: no rotation, cos / sin unused), d % 8 == 0, qkv and cache 16-byte aligned.
 MB_API int mb_rope_append(void* qkv, void* cache, const float* cosv, const float* sinv, int batch, int seq, int hq,
                           int hk, int d, int rot, int off, long cache_sb, int pdl, cudaStream_t stream) {
   if (rot % 16 || rot > d || d % 8 || cache_sb % 8) return -1;
+  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cache)) & 15) return -1;
   const long nvec = static_cast<long>(batch) * seq * (hq + 2 * hk) * (d / 8);
   if (!nvec) return 0;
   long blocks = (nvec + 255) / 256;

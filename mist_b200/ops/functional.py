@@ -735,7 +735,7 @@ def decode_attention(q, k_cache, v_cache, seq_len: int, scale: Optional[float] =
     nkv = k_cache.shape[2]
     scale = float(scale if scale is not None else 1.0 / math.sqrt(d))
     if not (use_native(q) and q.dtype == torch.bfloat16 and d % 8 == 0 and d <= 256
-            and k_cache.stride(3) == 1 and v_cache.stride(3) == 1
+            and k_cache.stride(3) == 1 and v_cache.stride(3) == 1 and (ptr(k_cache) | ptr(v_cache)) % 16 == 0
             and all(st % 8 == 0 for st in k_cache.stride()[:3] + v_cache.stride()[:3])):
         k = k_cache[:, :seq_len].float()
         v = v_cache[:, :seq_len].float()
@@ -744,8 +744,8 @@ def decode_attention(q, k_cache, v_cache, seq_len: int, scale: Optional[float] =
             v = v.repeat_interleave(nh // nkv, dim=2)
         s = torch.einsum("bhd,bkhd->bhk", q.float(), k) * scale
         return torch.einsum("bhk,bkhd->bhd", torch.softmax(s, dim=-1), v).to(q.dtype)
-    if q.stride(2) != 1 or q.stride(1) != d or q.stride(0) % 8:
-        q = q.contiguous()
+    if q.stride(2) != 1 or q.stride(1) != d or q.stride(0) % 8 or ptr(q) % 16:       # 16-byte loads
+        q = q.clone(memory_format=torch.contiguous_format)
     out = torch.empty(b, nh, d, dtype=q.dtype, device=q.device)
     ks, vs = k_cache.stride(), v_cache.stride()
     call("mb_decode_attn", ptr(q), ptr(k_cache), ptr(v_cache), ptr(out), b, nh, nkv, d, int(seq_len),
@@ -757,7 +757,7 @@ def rope_append_available(qkv, cache, rot: int, d: int) -> bool:
     """Whether :func:`rope_append_` may take ``qkv``; it works outside autograd, so not where a gradient is recorded."""
     recorded = torch.is_grad_enabled() and (qkv.requires_grad or cache.requires_grad)
     return (not _sym(qkv) and not recorded and use_native(qkv) and qkv.dtype == torch.bfloat16
-            and cache.dtype == torch.bfloat16 and d % 8 == 0 and rot % 16 == 0)
+            and cache.dtype == torch.bfloat16 and d % 8 == 0 and rot % 16 == 0 and (ptr(qkv) | ptr(cache)) % 16 == 0)
 
 
 def rope_append_(qkv, cache, offset: int, hq: int, hk: int, d: int, rotary=None):
