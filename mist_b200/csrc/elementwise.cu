@@ -509,6 +509,7 @@ MB_API int mb_cast_f32_to_bf16(const float* in, void* out, size_t n, float scale
 }
 MB_API int mb_add_f32_to_bf16(const float* src, void* dst, size_t n, cudaStream_t s) {
   if (!n) return 0;
+  if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) return -1;
   add_f32_to_bf16_kernel<<<grid_for((n + 7) / 8), kBlock, 0, s>>>(src, BFM(dst), n);
   return LAUNCH_OK();
 }

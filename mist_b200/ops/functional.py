@@ -1139,7 +1139,7 @@ class _EmbeddingFn(torch.autograd.Function):
         v0, v1 = ctx.v0, ctx.v0 + wte.shape[0]
         bucket = getattr(ctx.param, "grad_bucket", None) if use_native(wte) and ctx.needs_input_grad[1] else None
         accumulate = bool(getattr(ctx.param, "grad_accumulate", False))
-        if bucket is not None and bucket.dtype == torch.float32:      # summed in place
+        if bucket is not None and bucket.dtype == torch.float32 and bucket.is_contiguous():      # summed in place
             dwte = bucket if accumulate else bucket.zero_()
         else:
             dwte = torch.zeros(wte.shape, dtype=torch.float32, device=wte.device)
@@ -1160,7 +1160,9 @@ class _EmbeddingFn(torch.autograd.Function):
         if bucket is None:
             return None, dwte.to(wte.dtype), dwpe, None
         if dwte is not bucket:
-            if accumulate:
+            if bucket.dtype != torch.bfloat16 or not bucket.is_contiguous() or ptr(bucket) % 16:
+                bucket.add_(dwte) if accumulate else bucket.copy_(dwte)      # any type, order and start
+            elif accumulate:
                 call("mb_add_f32_to_bf16", ptr(dwte), ptr(bucket), dwte.numel(), stream())
             else:
                 cast_to_bf16(dwte, bucket)
