@@ -419,11 +419,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 // delta[b][h][q] = sum_d dO[b][q][h][d] * O[b][q][h][d]; sixteen lanes per (b, q, h), one vector each, and four rows at a
 // time so that eight loads of a thread are in flight.
 constexpr int kDeltaRows = 4;
+// First row of a thread.  Rows are counted in 32 bits, threads would not fit: 4 per row, of up to 2^31 - 1 rows.
+__host__ __device__ inline unsigned delta_first_row(unsigned block, unsigned thread) {
+  return (block * 16u + (thread >> 4)) * kDeltaRows;
+}
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o,
                   float* __restrict__ delta, int batch, int sq, int nh, int d, long do_bs,
                   long do_ts, long do_hs, long o_bs, long o_ts, long o_hs) {
-  const unsigned first = ((blockIdx.x * 256u + threadIdx.x) >> 4) * kDeltaRows;
+  const unsigned first = delta_first_row(blockIdx.x, threadIdx.x);
   const int sub = threadIdx.x & 15;
   const unsigned total = static_cast<unsigned>(batch) * sq * nh;
   mb::bf16x8 x[kDeltaRows], y[kDeltaRows];
@@ -560,6 +564,8 @@ MB_API int* mb_status_device_ptr();
 MB_API void mb_attn_bwd_set_variant(int v) { g_bwd_variant = (v == 1) ? 1 : 0; }
 // Variant the last call of mb_attn_bwd launched.
 MB_API int mb_attn_bwd_last_variant() { return g_bwd_last_variant; }
+// First of the rows of dO . O that a thread of a block sums (what the kernel computes, for checks on the host).
+MB_API unsigned mb_attn_delta_first_row(unsigned block, unsigned thread) { return delta_first_row(block, thread); }
 
 // dout, o: [b][sq][nh][d] with the given element strides for dout (o is contiguous);
 // delta: [b][nh][sq] fp32 scratch; dq_acc: [b][nh][sq][d] fp32 scratch, zeroed by this call.
