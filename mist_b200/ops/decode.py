@@ -93,6 +93,8 @@ def _stack(layers, hidden, residual):
         return None
     if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks:
         return None
+    if Settings.gemm_backend != "tcgen05" or Settings.gemm_max_ctas:       # the step's GEMMs know no limit
+        return None
     if residual is not None and (residual.dtype is not _BF16 or residual.shape != hidden.shape
                                  or residual.device != hidden.device):
         return None
@@ -130,8 +132,7 @@ def _rows(x):
 def stack_step(layers, hidden, residual):
     """``(hidden, residual)`` behind ``layers`` for one new token per sequence (``hidden`` ``[b, 1, h]``), with the
     caches of the blocks' ``inference_params`` extended by it; ``None`` when the general path is needed."""
-    if (not hidden.is_cuda or hidden.dtype is not _BF16 or torch.is_grad_enabled()
-            or Settings.gemm_backend != "tcgen05"):
+    if not hidden.is_cuda or hidden.dtype is not _BF16 or torch.is_grad_enabled():
         return None
     found = _stack(layers, hidden, residual)
     if found is None:

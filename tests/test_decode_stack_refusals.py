@@ -95,6 +95,14 @@ def test_batch_limit():
         assert decode._stack(layers, torch.zeros(129, 1, 64, dtype=BF16), None) is None
 
 
+@pytest.mark.parametrize("name,value", [("gemm_backend", "cublas"), ("gemm_max_ctas", 100)])
+def test_settings(name, value, monkeypatch):
+    net, layers = _model("cpu")
+    monkeypatch.setattr(decode.Settings, name, value)
+    with torch.no_grad(), kv_cache(net, 1, 2):
+        assert decode._stack(layers, torch.zeros(1, 1, 64, dtype=BF16), None) is None
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("change", ["forward", "global_hook"])
 def test_replaced_forwards_run(change):
