@@ -20,6 +20,7 @@ from typing import Optional
 
 import torch
 import torch.nn as nn
+from torch.nn.modules import module as nn_module
 
 from ..ops import functional as F
 from ..parallel import dist_ops
@@ -404,6 +405,15 @@ class ParallelMHA(nn.Module):
             outs.append(q_mask.restore(oi, i) if q_mask is not None else oi)
         return torch.cat(outs, 0)
 
+    def _own(self, qkv):
+        """``qkv``, the output of ``Wqkv``, contiguous and free to be written: the projection keeps its input and not its
+        output, but a hook or a replaced projection may hold on to it."""
+        m = self.Wqkv
+        if (type(m) is not ColumnParallelLinear or m._forward_hooks or "forward" in m.__dict__
+                or nn_module._global_forward_hooks):
+            return qkv.clone(memory_format=torch.contiguous_format)
+        return qkv.contiguous()
+
     def _forward_cached(self, x, residual=None):
         """Inference with a key/value cache (``self.inference_params`` set by
         :mod:`mist_b200.inference`): the new keys and values are appended to this layer's cache;
@@ -423,8 +433,10 @@ class ParallelMHA(nn.Module):
             cos, sin = F.rope_tables(ip.max_seqlen, self.rotary_emb_dim, self.rotary_emb_base, qkv.device)
             rotary = (cos[off:off + s], sin[off:off + s], self.rotary_emb_dim)
         cache = ip.cache_for(self.layer_idx, b, hk, d, qkv.dtype, qkv.device)      # [b, max_seq, 2, hk, d]
-        if F.rope_append_available(qkv, cache, self.rotary_emb_dim, d):
+        if qkv.is_contiguous() and F.rope_append_available(qkv, cache, self.rotary_emb_dim, d):
             assert off + s <= cache.shape[1], "sequence longer than the cache was sized for"
+            if rotary is not None:
+                qkv = self._own(qkv)
             F.rope_append_(qkv, cache, off, hq, hk, d, rotary)
             q = qkv[..., : hq * d].view(b, s, hq, d)
             k, v = cache[:b, off:off + s, 0], cache[:b, off:off + s, 1]
@@ -468,7 +480,8 @@ class ParallelMHA(nn.Module):
                 if self.rotary_emb_dim > 0:        # positions are those of the padded layout
                     rotary = (*F.rope_tables(s, self.rotary_emb_dim, self.rotary_emb_base, qkv.device),
                               self.rotary_emb_dim)
-                ctx = F.attention_projected(qkv.view(b, s, -1, self.head_dim), self.local_heads_kv, self.softmax_scale,
+                    qkv = self._own(qkv)           # rotated in place
+                ctx = F.attention_projected(qkv.reshape(b, s, -1, self.head_dim), self.local_heads_kv, self.softmax_scale,
                                             self.causal, rotary,
                                             None if attention_mask is None else attention_mask.lengths_dev)
             elif self.local_heads == self.local_heads_kv:
