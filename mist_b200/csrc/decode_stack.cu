@@ -116,7 +116,7 @@ struct Block {
 }  // namespace
 
 MB_API int mb_gemm_skinny_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                               int flags, const void* bias, const void* aux, float alpha, int pdl,
+                               int flags, const void* bias, const void* aux, float alpha, int always, int pdl,
                                cudaStream_t stream);
 MB_API int mb_decode_attn(const void* q, const void* k, const void* v, void* o, int batch, int nh, int nh_kv, int d,
                           int len, long q_sb, long k_sb, long k_ss, long k_sh, long v_sb, long v_ss, long v_sh,
@@ -163,18 +163,18 @@ MB_API int mb_decode_stack(const void* hidden, const void* residual, void* out_h
     // the residual stream alternates between res_mid (behind norm1) and out_residual (behind norm2)
     MB_STEP(launch_norm(x, res, b.norm1_w, b.norm1_b, z, res_mid, batch, h, eps, rms, i > 0, stream));
     MB_STEP(mb_gemm_skinny_bf16(z, b.wqkv, qkv, batch, static_cast<int>(qkv_cols), h, h, h, static_cast<int>(qkv_cols),
-                                b.bqkv ? 1 : 0, b.bqkv, nullptr, 1.f, 1, stream));
+                                b.bqkv ? 1 : 0, b.bqkv, nullptr, 1.f, 1, 1, stream));
     MB_STEP(mb_rope_append(qkv, b.cache, cosv, sinv, batch, 1, hq, hk, d, rot, off, cache_sb, 1, stream));
     const __nv_bfloat16* kc = static_cast<const __nv_bfloat16*>(b.cache);
     const __nv_bfloat16* vc = kc + static_cast<long>(hk) * d;
     MB_STEP(mb_decode_attn(qkv, kc, vc, ctx, batch, hq, hk, d, off + 1, qkv_cols, cache_sb, 2L * hk * d, d, cache_sb,
                            2L * hk * d, d, scale[i], 1, stream));
     MB_STEP(mb_gemm_skinny_bf16(ctx, b.wo, branch, batch, h, ctx_cols, ctx_cols, ctx_cols, h, b.bo ? 1 : 0, b.bo,
-                                nullptr, 1.f, 1, stream));
+                                nullptr, 1.f, 1, 1, stream));
     MB_STEP(launch_norm(branch, res_mid, b.norm2_w, b.norm2_b, z, out_residual, batch, h, eps, rms, 1, stream));
-    MB_STEP(mb_gemm_skinny_bf16(z, b.w1, act, batch, f, h, h, h, f, act_flags | (b.b1 ? 1 : 0), b.b1, nullptr, 1.f, 1,
+    MB_STEP(mb_gemm_skinny_bf16(z, b.w1, act, batch, f, h, h, h, f, act_flags | (b.b1 ? 1 : 0), b.b1, nullptr, 1.f, 1, 1,
                                 stream));
-    MB_STEP(mb_gemm_skinny_bf16(act, b.w2, out_hidden, batch, h, f, f, f, h, b.b2 ? 1 : 0, b.b2, nullptr, 1.f, 1,
+    MB_STEP(mb_gemm_skinny_bf16(act, b.w2, out_hidden, batch, h, f, f, f, h, b.b2 ? 1 : 0, b.b2, nullptr, 1.f, 1, 1,
                                 stream));
     x = out_hidden;
     res = out_residual;

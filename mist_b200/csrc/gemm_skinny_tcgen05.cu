@@ -8,7 +8,8 @@
 //   * the CTAs of a cluster (up to eight) share the K range of a tile and sum their fp32 partial tiles through
 //     distributed shared memory in rank order: enough CTAs for any N, one launch, no workspace, the same bits on
 //     every run;
-//   * four 18 - 24 KB stages and two or three CTAs per SM keep about 200 KB of W per SM in flight;
+//   * four stages keep W streaming: 18 - 24 KB each and two or three CTAs per SM up to 64 tokens (150 - 220 KB in
+//     flight), 32 KB each and one CTA per SM (128 KB) above;
 //   * W does not depend on the kernel before: launched as a programmatic dependent (`pdl`), the CTAs start to load W
 //     while that kernel drains and wait for it only before they read x.  The caller may ask for that only where no
 //     kernel still running can write W.
@@ -17,6 +18,7 @@
 // Reference counterpart: the cuBLAS calls of csrc/fused_dense_lib/fused_dense_cuda.cu:19-92 at small batch.
 #include "sm100_pair.cuh"
 #include <string.h>
+#include <type_traits>
 
 using namespace sm100;
 
@@ -56,9 +58,12 @@ struct SkinnyLayout {
 __device__ __forceinline__ void report(int* status, int code) {
   if (status) atomicCAS(status, 0, code);
 }
-__device__ __forceinline__ float2 ld_cluster2(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+// (volatile keeps the load behind the cluster barrier; without a memory clobber several can be in flight)
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr));
   return v;
 }
 
@@ -186,59 +191,91 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   __syncthreads();
   if (split > 1) cluster_sync_all();
 
-  // two neighbouring columns per thread; the CTAs of the cluster share the outputs
-  const int pairs = width / 2;
-  const uint32_t part_u = smem_u32(smem);
-  for (int t = rank * kThreads + threadIdx.x; t < p.M * pairs; t += split * kThreads) {
-    const int m = t / pairs, c = (t - m * pairs) * 2, n = n0 + c;
-    if (n >= p.N) continue;
-    const uint32_t off = part_u + static_cast<uint32_t>(m * L::kPartStride + c) * 4;
-    float2 v = make_float2(0.f, 0.f), u = make_float2(0.f, 0.f);
+  // Four neighbouring columns per thread, the same ones for all of its tokens; the CTAs of the cluster take the tokens in
+  // turn.
+  // The loads of two tokens (and of all parts) are issued before the first sum: with one pair of columns at a time a
+  // tile of 128 tokens spent 12 us here, 280 ns an output.
+  const int quads = width / 4;                             // 32, or 16 for SwiGLU: both divide the threads
+  const int c = (threadIdx.x % quads) * 4, n = n0 + c;
+  const int live = min(4, p.N - n);                        // columns that exist; may be negative
+  const int m_step = split * (kThreads / quads);
+  if (live > 0) {
+    float bias[4] = {0.f, 0.f, 0.f, 0.f}, bias_up[4] = {0.f, 0.f, 0.f, 0.f};
+    if (p.flags & EPI_BIAS) {
 #pragma unroll
-    for (int r = 0; r < kMaxSplit; ++r) {
-      if (r < split) {
-        const uint32_t at = split > 1 ? map_to_cta(off, r) : off;
-        const float2 a = ld_cluster2(at);
-        v.x += a.x;
-        v.y += a.y;
-        if (swiglu) {
-          const float2 b = ld_cluster2(at + (BR / 2) * 4);
-          u.x += b.x;
-          u.y += b.y;
+      for (int i = 0; i < 4; ++i) {
+        if (i < live) {
+          bias[i] = __bfloat162float(p.bias[n + i]);
+          if (swiglu) bias_up[i] = __bfloat162float(p.bias[p.N + n + i]);
         }
       }
     }
-    v.x *= p.alpha;
-    v.y *= p.alpha;
-    u.x *= p.alpha;
-    u.y *= p.alpha;
-    const bool two = n + 1 < p.N;
-    if (p.flags & EPI_BIAS) {
-      v.x += __bfloat162float(p.bias[n]);
-      if (two) v.y += __bfloat162float(p.bias[n + 1]);
-      if (swiglu) {
-        u.x += __bfloat162float(p.bias[p.N + n]);
-        if (two) u.y += __bfloat162float(p.bias[p.N + n + 1]);
+    const bool wide = live == 4 && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 7) == 0;
+    const float* part = reinterpret_cast<const float*>(smem) + c;
+    const uint32_t part_u = smem_u32(part);
+    constexpr int U = 2;
+    for (int m0 = rank + split * (threadIdx.x / quads); m0 < p.M; m0 += U * m_step) {
+      float v[U][4], up[U][4];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int m = m0 + u * m_step;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (m >= p.M) {
+        } else if (split == 1) {
+          const float* at = part + m * L::kPartStride;
+          a = *reinterpret_cast<const float4*>(at);
+          if (swiglu) b = *reinterpret_cast<const float4*>(at + BR / 2);
+        } else {
+          const uint32_t off = part_u + static_cast<uint32_t>(m * L::kPartStride) * 4;
+          float4 x[kMaxSplit], y[kMaxSplit];
+#pragma unroll
+          for (int r = 0; r < kMaxSplit; ++r) {
+            x[r] = y[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < split) {
+              const uint32_t at = map_to_cta(off, r);
+              x[r] = ld_cluster4(at);
+              if (swiglu) y[r] = ld_cluster4(at + (BR / 2) * 4);
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < kMaxSplit; ++r) {
+            a.x += x[r].x; a.y += x[r].y; a.z += x[r].z; a.w += x[r].w;
+            b.x += y[r].x; b.y += y[r].y; b.z += y[r].z; b.w += y[r].w;
+          }
+        }
+        v[u][0] = a.x; v[u][1] = a.y; v[u][2] = a.z; v[u][3] = a.w;
+        up[u][0] = b.x; up[u][1] = b.y; up[u][2] = b.z; up[u][3] = b.w;
       }
-    }
-    if (p.flags & EPI_GELU) {
-      v.x = mb::gelu_tanh(v.x);
-      v.y = mb::gelu_tanh(v.y);
-    }
-    if (swiglu) {
-      v.x = mb::silu(v.x) * u.x;
-      v.y = mb::silu(v.y) * u.y;
-    }
-    const long o = static_cast<long>(m) * p.ldc + n;
-    if (p.flags & EPI_RESIDUAL) {
-      v.x += __bfloat162float(p.aux[o]);
-      if (two) v.y += __bfloat162float(p.aux[o + 1]);
-    }
-    if (two && (p.ldc & 1) == 0)
-      *reinterpret_cast<__nv_bfloat162*>(p.C + o) = __floats2bfloat162_rn(v.x, v.y);
-    else {
-      p.C[o] = __float2bfloat16(v.x);
-      if (two) p.C[o + 1] = __float2bfloat16(v.y);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int m = m0 + u * m_step;
+        if (m >= p.M) break;
+        const long o = static_cast<long>(m) * p.ldc + n;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float x = v[u][i] * p.alpha;
+          if (p.flags & EPI_BIAS) x += bias[i];
+          if (p.flags & EPI_GELU) x = mb::gelu_tanh(x);
+          if (swiglu) {
+            float y = up[u][i] * p.alpha;
+            if (p.flags & EPI_BIAS) y += bias_up[i];
+            x = mb::silu(x) * y;
+          }
+          if ((p.flags & EPI_RESIDUAL) && i < live) x += __bfloat162float(p.aux[o + i]);
+          v[u][i] = x;
+        }
+        if (wide) {
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(v[u][0], v[u][1]), hi = __floats2bfloat162_rn(v[u][2], v[u][3]);
+          uint2 w;
+          w.x = *reinterpret_cast<const uint32_t*>(&lo);
+          w.y = *reinterpret_cast<const uint32_t*>(&hi);
+          *reinterpret_cast<uint2*>(p.C + o) = w;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (i < live) p.C[o + i] = __float2bfloat16(v[u][i]);
+        }
+      }
     }
   }
   if (split > 1) cluster_sync_all();      // nobody leaves while its partial tile is being read
@@ -279,29 +316,61 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
 }
 
 template <int NT>
-int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int tiles, int split, int pdl,
-                  cudaStream_t stream) {
-  constexpr int smem = SkinnyLayout<NT>::kTotal + 1024;
-  auto kern = gemm_skinny_kernel<NT>;
-  static const bool configured =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
-  if (!configured) return -3;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(split, tiles, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+void skinny_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int tiles, int split, cudaStream_t stream) {
+  memset(cfg, 0, sizeof(*cfg));
+  cfg->gridDim = dim3(split, tiles, 1);
+  cfg->blockDim = dim3(kThreads, 1, 1);
+  cfg->dynamicSmemBytes = SkinnyLayout<NT>::kTotal + 1024;
+  cfg->stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = split;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+}
+template <int NT>
+bool configure() {
+  static const bool ok = cudaFuncSetAttribute(gemm_skinny_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              SkinnyLayout<NT>::kTotal + 1024) == cudaSuccess;
+  return ok;
+}
+// SMs that clusters of a size can occupy together, one CTA on each (cudaOccupancyMaxActiveClusters on a B200: the CTAs of
+// a cluster share a GPC).  A constant, so that sums are cut the same way on every GPU.
+constexpr int kClusterSms[kMaxSplit + 1] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
+
+// CTAs that share a tile's K range: as many as leave each at least four K blocks (one ring) and the whole grid resident
+// (three CTAs per SM with 16 columns, one with 128, whose stages are larger): a second wave costs more than shorter sums
+// give.  7680 x 2560 at 32 tokens (60 tiles): 4 CTAs a tile 11.7 us, 8 CTAs 19.4; 12288 x 4096 (96 tiles, at most 90
+// clusters of three): 2 CTAs a tile 22.4 us, 3 CTAs 29.0; 22016 x 4096 at one token (172 tiles): 2 CTAs a tile 31.2 us,
+// one 33.8.
+template <int NT>
+int choose_split(int tiles, int num_kb) {
+  constexpr int per_sm = NT == 16 ? 3 : NT <= 64 ? 2 : 1;
+  int split = num_kb / 4 < kMaxSplit ? num_kb / 4 : kMaxSplit;
+  while (split > 1 && kClusterSms[split] / split * per_sm < tiles) --split;
+  return split < 1 ? 1 : split;
+}
+
+// Whether this kernel beats the tiled ones, which put the tokens on the 128-row side of the product; both sides measured
+// for N from 64 to 50304 and K from 64 to 50304.  Up to 32 tokens it does at every size (0.14 - 0.96 of their time).
+// Above, its epilogue needs enough K blocks to hide behind: at 64 tokens 512 x 512 took 7.5 us against 6.7 and
+// 50304 x 1024 28.9 against 28.1, but 1024 x 1024 7.0 against 8.9.  Above 64 its stages leave one CTA per SM, and it has
+// to split K to win: 128 tokens, 4096 x 4096 16 us against 24, but 12288 x 4096 31 against 26.
+bool pays(int M, int num_kb, int split) {
+  return M <= 32 || (split > 1 && num_kb >= 16) || (M <= 64 && num_kb >= 32);
+}
+
+template <int NT>
+int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int tiles, int split, int pdl,
+                  cudaStream_t stream) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  skinny_config<NT>(&cfg, attr, tiles, split, stream);
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, tw, tx, p) == cudaSuccess ? 0 : -4;
+  return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NT>, tw, tx, p) == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace
@@ -310,9 +379,10 @@ MB_API int* mb_status_device_ptr();
 
 // C[M, N] = epi(alpha * A[M, K] B[N, K]^T) for M <= 128, bf16 in and out.  flags: bias, GELU, residual (aux, row
 // stride ldc), or 128: SwiGLU, where B holds 2 N rows [gate | up] (and the bias 2 N values).  A and B 16-byte
-// aligned, lda and ldb multiples of 8.  Returns 1 without launching when the arguments need another kernel.
+// aligned, lda and ldb multiples of 8.  Returns 1 without launching when the arguments need another kernel or, unless
+// `always`, when another one is faster.
 MB_API int mb_gemm_skinny_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                               int flags, const void* bias, const void* aux, float alpha, int pdl,
+                               int flags, const void* bias, const void* aux, float alpha, int always, int pdl,
                                cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
@@ -326,14 +396,6 @@ MB_API int mb_gemm_skinny_bf16(const void* A, const void* B, void* C, int M, int
   const int tiles = (N + width - 1) / width;
   if (tiles > 65535) return 1;
   const int num_kb = (K + BK - 1) / BK;
-  const int nt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-  // CTAs that share a tile's K range: doubled while the grid has fewer than two CTAs per SM and a CTA keeps at
-  // least four k-blocks (one ring).
-  int split = 1;
-  while (split < kMaxSplit && static_cast<long>(tiles) * split < 2L * 148 && num_kb >= 8 * split) split *= 2;
-  CUtensorMap tw, tx;
-  if (!make_map(&tw, B, static_cast<uint64_t>(N) * (swiglu ? 2 : 1), K, ldb, BR / 2)) return -2;
-  if (!make_map(&tx, A, M, K, lda, nt)) return -2;
   SkinnyParams p;
   p.M = M; p.N = N; p.K = K;
   p.C = reinterpret_cast<__nv_bfloat16*>(C);
@@ -343,8 +405,18 @@ MB_API int mb_gemm_skinny_bf16(const void* A, const void* B, void* C, int M, int
   p.flags = flags;
   p.alpha = alpha;
   p.status = mb_status_device_ptr();
-  if (nt == 16) return launch_skinny<16>(tw, tx, p, tiles, split, pdl, stream);
-  if (nt == 32) return launch_skinny<32>(tw, tx, p, tiles, split, pdl, stream);
-  if (nt == 64) return launch_skinny<64>(tw, tx, p, tiles, split, pdl, stream);
-  return launch_skinny<128>(tw, tx, p, tiles, split, pdl, stream);
+  auto run = [&](auto nt) -> int {
+    constexpr int NT = decltype(nt)::value;
+    if (!configure<NT>()) return -3;
+    const int split = choose_split<NT>(tiles, num_kb);
+    if (!always && !pays(M, num_kb, split)) return 1;
+    CUtensorMap tw, tx;
+    if (!make_map(&tw, B, static_cast<uint64_t>(N) * (swiglu ? 2 : 1), K, ldb, BR / 2)) return -2;
+    if (!make_map(&tx, A, M, K, lda, NT)) return -2;
+    return launch_skinny<NT>(tw, tx, p, tiles, split, pdl, stream);
+  };
+  if (M <= 16) return run(std::integral_constant<int, 16>());
+  if (M <= 32) return run(std::integral_constant<int, 32>());
+  if (M <= 64) return run(std::integral_constant<int, 64>());
+  return run(std::integral_constant<int, 128>());
 }

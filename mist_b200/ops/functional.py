@@ -113,9 +113,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         flags |= EPI_BIAS
     if (M <= 128 and tile_n == 0 and not a_mn and not b_mn and out.dtype == torch.bfloat16
             and not Settings.gemm_max_ctas):       # that kernel takes the whole chip
-        # a few tokens: the kernel that puts W on the 128-row side and splits K (1: epilogue not covered)
+        # a few tokens: the kernel that puts W on the 128-row side and splits K (1: epilogue not covered, or slower)
         rc = native.kernels().mb_gemm_skinny_bf16(ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0),
-                                                  out.stride(0), flags, ptr(bias), ptr(aux), float(alpha), 0, stream())
+                                                  out.stride(0), flags, ptr(bias), ptr(aux), float(alpha), 0, 0, stream())
         if rc == 0:
             native.launch_count += 1
             return out

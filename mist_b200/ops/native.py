@@ -38,7 +38,7 @@ _SIGNATURES = {
     "mb_gemm_pair_bf16": ([_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p, _p, _f, _i, _p], _i),
     "mb_decode_attn": ([_p, _p, _p, _p, _i, _i, _i, _i, _i, _l, _l, _l, _l, _l, _l, _l, _f, _i, _p], _i),
     "mb_rope_append": ([_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _l, _i, _p], _i),
-    "mb_gemm_skinny_bf16": ([_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p, _p, _f, _i, _p], _i),
+    "mb_gemm_skinny_bf16": ([_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p, _p, _f, _i, _i, _p], _i),
     "mb_decode_stack_scratch": ([_i, _i, _i, _i, _i, _i], _l),
     "mb_decode_stack": ([_p] * 5 + [_i, _p] + [_i] * 8 + [_f, _p, _p, _p, _i, _i, _l, _p], _i),
     "mb_norm_bwd_scratch_rows": ([_i, _i], _i),

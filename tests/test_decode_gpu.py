@@ -69,6 +69,39 @@ def test_skinny_gemm(M, N, K):
     assert _rel(F.gemm(x, w, bias=bias, flags=F.EPI_GELU), act) < 2 ** -8
 
 
+# The kernel itself, also where another one is faster: K for one to eight CTAs per tile (four K blocks each), a K tail,
+# rows of one token, of whole rounds of tokens and one more; C rows that allow 8-byte, 4-byte and 2-byte stores
+@pytest.mark.parametrize("M", [1, 6, 16, 17, 33, 65, 128])
+@pytest.mark.parametrize("N,K,ldc", [(192, 64, 192), (128, 520, 128), (320, 768, 324), (128, 1024, 130),
+                                     (128, 1280, 131), (64, 1536, 64), (128, 1800, 128), (448, 2048, 450)])
+@pytest.mark.parametrize("epi", ["plain", "gelu", "residual", "swiglu", "swiglu_bias"])
+def test_skinny_kernel(M, N, K, ldc, epi):
+    from mist_b200.ops import native
+    torch.manual_seed(N + K)
+    swiglu = epi.startswith("swiglu")
+    rows = 2 * N if swiglu else N
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(rows, K, device=DEV, dtype=torch.bfloat16) * K ** -0.5
+    bias = torch.randn(rows, device=DEV, dtype=torch.bfloat16)
+    aux = torch.randn(M, ldc, device=DEV, dtype=torch.bfloat16)
+    out = torch.full((M, ldc), 7.0, device=DEV, dtype=torch.bfloat16)
+    flags = {"plain": 0, "gelu": F.EPI_BIAS | F.EPI_GELU, "residual": F.EPI_RESIDUAL, "swiglu": 128,
+             "swiglu_bias": 128 | F.EPI_BIAS}[epi]
+    native.call("mb_gemm_skinny_bf16", x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, ldc, flags,
+                bias.data_ptr(), aux.data_ptr(), 1.0, 1, 0, native.stream())
+    ref = x.double() @ w.double().t() + (bias.double() if flags & F.EPI_BIAS else 0)
+    if epi == "gelu":
+        ref = torch.nn.functional.gelu(ref, approximate="tanh")
+    elif epi == "residual":
+        ref = ref + aux[:, :N].double()
+    elif swiglu:
+        ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
+    # fp32 sums and one rounding to bf16 (2^-9 of a value at most); the activations add the error of their exponential
+    # (2^-11)
+    assert _rel(out[:, :N], ref) < (2 ** -9 if epi in ("plain", "residual") else 2 ** -8)
+    assert (out[:, N:] == 7).all()
+
+
 @pytest.mark.parametrize("model,extra", [("gpt2/1.3b", []), ("llama/1.3b", []), ("llama/1.3b", ["model.num_heads_kv=2"])])
 @pytest.mark.parametrize("b", [1, 5, 40])
 def test_native_decode_step_matches_the_modules(model, extra, b, monkeypatch):
