@@ -5,7 +5,8 @@
 //
 // Bound: reading the cache once; there is no tensor-core work in a 1 x len product.  One CTA per (head, sequence)
 // reached 0.17 TB/s on one sequence of 2048 positions (32 CTAs, one position in flight per warp: 193 us) and
-// 1.6 TB/s on 32 sequences of 1000 (201 us); this kernel takes 13 us and 87 us (3.8 TB/s).  Here
+// 1.6 TB/s on 32 sequences of 1000 (32 heads of 80; 201 us); this kernel takes 9.7 us and 57 us (5.7 TB/s), the other
+// remains for short sequences (see short_is_faster).  Here
 //   * a cluster of up to eight CTAs shares the positions of one (head, sequence) and merges its partial
 //     (max, sum, output) triples through distributed shared memory: enough CTAs for one sequence, one launch,
 //     no workspace;
@@ -19,6 +20,9 @@
 //     summed over the lanes together (each round halves what a lane still holds; a lane ends up with one score, one
 //     maximum and one exponential per stage, and the four probabilities are handed out by shuffles), products run on
 //     packed fp32 pairs, and the piece addresses advance by a constant;
+//   * two CTAs fit an SM at every head size: what is merged lies over the ring, and a short chunk takes only the stages
+//     that it fills.  With arrays of their own, and four stages at head size 64, one CTA fitted: 32 x 1000 positions of
+//     32 heads of 128 on 8 took 119 us, now 32; 16 x 130 positions of 32 heads of 64 58 us, now 8.7;
 //   * query heads that share a key/value head (grouped-query attention) go through one CTA in groups of up to
 //     four, so the cache is read once per group of four instead of once per query head.
 //
@@ -53,19 +57,25 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool real)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(real ? 16 : 0) : "memory");
 }
 
+// Maxima, sums and weighted values of the warps (s_) and of the CTA (c_).
+template <int LPP, int G>
+struct MergeArrays {
+  float s_acc[kWarps][G][LPP * 8], c_acc[G][LPP * 8];
+  float s_m[kWarps][G], s_l[kWarps][G], c_m[G], c_l[G];
+};
+
 // LPP lanes hold one position (a power of two >= d / 8), G query heads share the CTA.
 template <int LPP, int G, int STAGES>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, __nv_bfloat16* o, int nh,
-                   int group, int d, int len, int chunk, long q_sb, long k_sb, long k_ss, long k_sh, long v_sb,
-                   long v_ss, long v_sh, float scale_log2) {
+                   int group, int d, int len, int chunk, int stages, long q_sb, long k_sb, long k_ss, long k_sh,
+                   long v_sb, long v_ss, long v_sh, float scale_log2) {
   constexpr int PPW = 32 / LPP;
   constexpr int NP = PPW * kUnroll;         // positions per stage of a warp
   extern __shared__ __align__(16) uint8_t ring[];
-  __shared__ float s_m[kWarps][G], s_l[kWarps][G];
-  __shared__ float s_acc[kWarps][G][LPP * 8];
-  __shared__ float c_m[G], c_l[G];
-  __shared__ float c_acc[G][LPP * 8];
+  // what is merged lies over the ring, once every warp has read its positions
+  using Merge = MergeArrays<LPP, G>;
+  Merge& sm = *reinterpret_cast<Merge*>(ring);
 
   const int split = blockIdx.x, nsplit = gridDim.x;
   const int h0 = blockIdx.y * G, b = blockIdx.z;
@@ -91,7 +101,8 @@ decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bf
   const int j0 = split * chunk, j1 = min(len, j0 + chunk);
   const int vph = d >> 3;                                     // 16-byte pieces of one head
   const int stage_elems = 2 * NP * d;                         // K rows, then V rows
-  const __nv_bfloat16* wring = reinterpret_cast<const __nv_bfloat16*>(ring) + warp * STAGES * stage_elems;
+  // [warp][stage]: a chunk that takes fewer than STAGES stages has only those, and never reaches a later one
+  const __nv_bfloat16* wring = reinterpret_cast<const __nv_bfloat16*>(ring) + warp * stages * stage_elems;
   const uint32_t wring_u = sm100::smem_u32(wring);
   const int first = j0 + warp * NP;
   // the pieces this lane copies: NP * vph of K and as many of V, at most four of each per lane
@@ -221,6 +232,7 @@ decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bf
   }
 
   // positions of a warp -> one triple per warp -> one per CTA -> (cluster) one per query head
+  __syncthreads();
 #pragma unroll
   for (int g = 0; g < G; ++g) {
     l[g] += __shfl_xor_sync(0xffffffffu, l[g], O1);
@@ -247,12 +259,12 @@ decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bf
       m[g] = mn;
     }
     if (lane == 0) {
-      s_m[warp][g] = m[g];
-      s_l[warp][g] = l[g];
+      sm.s_m[warp][g] = m[g];
+      sm.s_l[warp][g] = l[g];
     }
     if (sub == 0) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) s_acc[warp][g][e0 + i] = o8[i];
+      for (int i = 0; i < 8; ++i) sm.s_acc[warp][g][e0 + i] = o8[i];
     }
   }
   __syncthreads();
@@ -260,22 +272,22 @@ decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bf
     const int g = t / d, e = t - g * d;
     float M = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, s_m[w][g]);
+    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, sm.s_m[w][g]);
     const float mr = (M == -INFINITY) ? 0.f : M;
     float L = 0.f, out = 0.f;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const float f = exp2f(s_m[w][g] - mr);
-      L += s_l[w][g] * f;
-      out += s_acc[w][g][e] * f;
+      const float f = exp2f(sm.s_m[w][g] - mr);
+      L += sm.s_l[w][g] * f;
+      out += sm.s_acc[w][g][e] * f;
     }
     if (nsplit == 1) {
       o[(static_cast<long>(b) * nh + h0 + g) * d + e] = __float2bfloat16(L > 0.f ? out / L : 0.f);
     } else {
-      c_acc[g][e] = out;
+      sm.c_acc[g][e] = out;
       if (e == 0) {
-        c_m[g] = M;
-        c_l[g] = L;
+        sm.c_m[g] = M;
+        sm.c_l[g] = L;
       }
     }
   }
@@ -287,7 +299,7 @@ decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bf
     float ms[kMaxSplit], M = -INFINITY;
 #pragma unroll
     for (int r = 0; r < kMaxSplit; ++r) {
-      ms[r] = r < nsplit ? ld_cluster(&c_m[g], r) : -INFINITY;
+      ms[r] = r < nsplit ? ld_cluster(&sm.c_m[g], r) : -INFINITY;
       M = fmaxf(M, ms[r]);
     }
     float L = 0.f, out = 0.f;
@@ -295,8 +307,8 @@ decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bf
     for (int r = 0; r < kMaxSplit; ++r) {
       if (r < nsplit) {
         const float f = exp2f(ms[r] - M);      // M is finite: position 0 belongs to the first CTA
-        L += ld_cluster(&c_l[g], r) * f;
-        out += ld_cluster(&c_acc[g][e], r) * f;
+        L += ld_cluster(&sm.c_l[g], r) * f;
+        out += ld_cluster(&sm.c_acc[g][e], r) * f;
       }
     }
     o[(static_cast<long>(b) * nh + h0 + g) * d + e] = __float2bfloat16(L > 0.f ? out / L : 0.f);
@@ -304,25 +316,123 @@ decode_attn_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bf
   sm100::cluster_sync_all();      // nobody leaves while its shared memory is being read
 }
 
+// Short sequences: a CTA per (query head, sequence), a warp per position, loads straight into registers.  What counts
+// there is how many CTAs an SM holds and how little one of them costs, not the bytes in flight.
+__global__ void __launch_bounds__(kWarps * 32)
+decode_attn_short_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, __nv_bfloat16* o,
+                         int nh, int group, int d, int len, long q_sb, long k_sb, long k_ss, long k_sh, long v_sb,
+                         long v_ss, long v_sh, float scale_log2) {
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int e0 = lane * 8;
+  const bool live = e0 < d;                 // d is a multiple of 8, so a lane is all in or all out
+  const int hk = h / group;
+  mb::let_next_kernel_start();
+  mb::wait_for_previous_kernel();
+
+  float qf[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (live) mb::unpack8(*reinterpret_cast<const mb::bf16x8*>(q + b * q_sb + static_cast<long>(h) * d + e0), qf);
+  const __nv_bfloat16* kb = k + b * k_sb + hk * k_sh + e0;
+  const __nv_bfloat16* vb = v + b * v_sb + hk * v_sh + e0;
+
+  float m = -INFINITY, l = 0.f;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int j = warp; j < len; j += kWarps) {
+    float kf[8], vf[8], dot = 0.f;
+    if (live) {
+      mb::unpack8(*reinterpret_cast<const mb::bf16x8*>(kb + j * k_ss), kf);
+      mb::unpack8(*reinterpret_cast<const mb::bf16x8*>(vb + j * v_ss), vf);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dot += qf[i] * kf[i];
+    }
+    dot = mb::warp_sum(dot) * scale_log2;           // every lane gets the full score (log2 domain)
+    const float m_new = fmaxf(m, dot);
+    const float m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+    const float corr = exp2f(m - m_ref);            // 2^-inf = 0 on the first position
+    const float p = exp2f(dot - m_ref);
+    l = l * corr + p;
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = acc[i] * corr + p * vf[i];
+    }
+    m = m_new;
+  }
+
+  __shared__ float s_m[kWarps], s_l[kWarps];
+  __shared__ float s_acc[kWarps][kMaxD];
+  if (lane == 0) {
+    s_m[warp] = m;
+    s_l[warp] = l;
+  }
+  if (live) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s_acc[warp][e0 + i] = acc[i];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < d; e += kWarps * 32) {
+    float M = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, s_m[w]);
+    const float mr = (M == -INFINITY) ? 0.f : M;
+    float L = 0.f, out = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float f = exp2f(s_m[w] - mr);            // 0 for a warp that saw no position
+      L += s_l[w] * f;
+      out += s_acc[w][e] * f;
+    }
+    o[(static_cast<long>(b) * nh + h) * d + e] = __float2bfloat16(L > 0.f ? out / L : 0.f);
+  }
+}
+
+// Where the short kernel is the faster one; both measured for head sizes 32 - 256, 1 - 96 sequences of 4 - 80 positions
+// and one, two and four query heads per CTA of the streaming kernel.  At 12 positions the two meet for one head per CTA.
+// More CTAs than are resident at once favour the lighter one for longer (48 x 32 heads of 64: the streaming kernel takes
+// 1.54 times as long at 16 positions, 1.01 at 32), and so do few CTAs of four heads, whose steps take four times as long
+// (4 x 16 heads of 256 on 4: 1.35 times at 16 positions, 1.14 at 80).
+bool short_is_faster(long heads, int group, int d, int len) {
+  if (group % 4 == 0) return len <= (heads / 4 > 128 ? 12 : d > 128 ? 96 : 32);
+  if (group % 2 == 0) return len <= 16;
+  return len <= (heads > 296 ? 40 : 12);
+}
+
+// CTAs that share the positions of a (head, sequence): what makes the waves of 296 CTAs (two per SM) cheapest, where a
+// CTA costs as much as reading 9600 / d positions (3 us) before its first one and a merge a third of that.  A CTA keeps
+// at least 32 positions.  (Doubled up to six waves, 16 x 130 positions of 32 heads of 64 ran as 2048 CTAs of 33 positions.)
+int choose_split(long ctas, int len, int d) {
+  const long fixed = 9600 / d;
+  int best = 1;
+  long best_cost = (ctas + 295) / 296 * (fixed + len);
+  for (int split = 2; split <= kMaxSplit && len >= 32 * split; split *= 2) {
+    const long cost = (ctas * split + 295) / 296 * (fixed + fixed / 3 + (len + split - 1) / split);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = split;
+    }
+  }
+  return best;
+}
+
 template <int LPP, int G, int STAGES>
 int launch_decode(const void* q, const void* k, const void* v, void* o, int batch, int nh, int group, int d, int len,
                   long q_sb, long k_sb, long k_ss, long k_sh, long v_sb, long v_ss, long v_sh, float scale_log2,
                   int pdl, cudaStream_t stream) {
-  // Split the positions while the grid is below six waves of two CTAs per SM (an uneven last wave costs little then)
-  // and a CTA keeps at least 32 positions, below which the merge outweighs the work.
-  const long ctas = static_cast<long>(batch) * (nh / G);
-  int split = 1;
-  while (split < kMaxSplit && ctas * split < 148L * 12 && len >= 64 * split) split *= 2;
+  const int split = choose_split(static_cast<long>(batch) * (nh / G), len, d);
   const int chunk = (len + split - 1) / split;
+  // stages beyond the ones that a chunk fills would only keep other CTAs away
+  const int stage_positions = kWarps * (32 / LPP * kUnroll);
+  const int steps = (chunk + stage_positions - 1) / stage_positions;
+  const int stages = steps < STAGES ? steps : STAGES;
+  const size_t ring = static_cast<size_t>(stages) * stage_positions * 2 * d * 2;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(split, nh / G, batch);
   cfg.blockDim = dim3(kWarps * 32, 1, 1);
-  cfg.dynamicSmemBytes = static_cast<size_t>(kWarps) * STAGES * 2 * (32 / LPP * kUnroll) * d * 2;
+  cfg.dynamicSmemBytes = ring > sizeof(MergeArrays<LPP, G>) ? ring : sizeof(MergeArrays<LPP, G>);
   cfg.stream = stream;
   auto kern = decode_attn_kernel<LPP, G, STAGES>;
   static const bool configured =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) == cudaSuccess;
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) == cudaSuccess;
   if (!configured) return -3;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -333,7 +443,7 @@ int launch_decode(const void* q, const void* k, const void* v, void* o, int batc
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, BF(q), BF(k), BF(v), BFM(o), nh, group, d, len, chunk,
+  return cudaLaunchKernelEx(&cfg, kern, BF(q), BF(k), BF(v), BFM(o), nh, group, d, len, chunk, stages,
                             q_sb, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh, scale_log2) == cudaSuccess
              ? 0
              : -4;
@@ -400,7 +510,8 @@ MB_API int mb_decode_attn(const void* q, const void* k, const void* v, void* o, 
   if (batch <= 0 || nh <= 0) return 0;
   if (d % 8 || d > kMaxD || d <= 0 || nh_kv <= 0 || nh % nh_kv || len < 1) return -1;
   if ((q_sb | k_sb | k_ss | k_sh | v_sb | v_ss | v_sh) & 7) return -1;
-  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) return -1;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15)
+    return -1;
   const int group = nh / nh_kv;
   const float sl = scale * 1.4426950408889634f;
 #define MB_DECODE(L_, G_, S_)                                                                                        \
@@ -412,8 +523,25 @@ MB_API int mb_decode_attn(const void* q, const void* k, const void* v, void* o, 
     if (group % 2 == 0) MB_DECODE(L_, 2, S_); \
     MB_DECODE(L_, 1, S_);                     \
   } while (0)
-  // stages per warp: four up to head size 96, three above (two CTAs of 96 KB per SM)
-  if (d <= 64) MB_DECODE_G(8, 4);
+  if (short_is_faster(static_cast<long>(batch) * nh, group, d, len)) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(nh, batch, 1);
+    cfg.blockDim = dim3(kWarps * 32, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, decode_attn_short_kernel, BF(q), BF(k), BF(v), BFM(o), nh, group, d, len, q_sb,
+                              k_sb, k_ss, k_sh, v_sb, v_ss, v_sh, sl) == cudaSuccess
+               ? 0
+               : -4;
+  }
+  // stages per warp: four where two CTAs of them fit an SM, else three (up to 96 KB per CTA)
+  if (d <= 48) MB_DECODE_G(8, 4);
+  if (d <= 64) MB_DECODE_G(8, 3);
   if (d <= 96) MB_DECODE_G(16, 4);
   if (d <= 128) MB_DECODE_G(16, 3);
   MB_DECODE_G(32, 3);

@@ -27,6 +27,22 @@ def test_decode_attention_splits(nh, nkv, d, seq_len):
     assert _rel(out.cpu(), ref) < 2 ** -9
 
 
+# both sides of the lengths at which another kernel takes over, for few and for many heads; one stage of the ring, two and
+# all of them, and lengths that make two, four and eight CTAs share a sequence
+@pytest.mark.parametrize("b,nh,nkv,d", [(1, 2, 2, 64), (10, 32, 32, 64), (2, 6, 3, 40), (3, 8, 2, 128), (33, 16, 4, 80),
+                                        (2, 8, 2, 256), (9, 5, 1, 136), (40, 8, 8, 16)])
+@pytest.mark.parametrize("seq_len", [1, 12, 13, 16, 17, 32, 33, 40, 41, 96, 97, 129, 200, 257, 600, 1100])
+def test_decode_attention_kernels(b, nh, nkv, d, seq_len):
+    torch.manual_seed(seq_len)
+    cache = torch.randn(b, seq_len + 2, 2, nkv, d, device=DEV, dtype=torch.bfloat16)
+    q = torch.randn(b, nh, d, device=DEV, dtype=torch.bfloat16)
+    cache[:, seq_len:] = float("nan")                 # what lies behind the last position takes no part
+    out = F.decode_attention(q, cache[:, :, 0], cache[:, :, 1], seq_len)
+    k, v = (cache[:, :seq_len, i].double().repeat_interleave(nh // nkv, 2) for i in (0, 1))
+    p = torch.softmax(torch.einsum("bhd,bkhd->bhk", q.double(), k) / d ** 0.5, -1)
+    assert _rel(out, torch.einsum("bhk,bkhd->bhd", p, v)) < 2 ** -9          # one rounding to bf16
+
+
 @pytest.mark.parametrize("hq,hk,d,rot,s", [(4, 4, 64, 64, 1), (8, 2, 128, 32, 7), (4, 4, 80, 16, 33), (6, 3, 80, 0, 5)])
 def test_rope_append(hq, hk, d, rot, s):
     torch.manual_seed(s)
