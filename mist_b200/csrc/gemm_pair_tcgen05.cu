@@ -68,11 +68,16 @@ __device__ __forceinline__ void report(int* status, int code) {
   if (status) atomicCAS(status, 0, code);
 }
 
-template <bool A_MN, bool B_MN, bool AUX>
+// What a kernel's epilogue does beside the common part.  The split form is a kernel of its own: its second source of the
+// products cost the others 4 - 9 % where the epilogue is the bound (13760 x 6664 x 128: 81.7 us against 87.4).
+enum Kind : int { kPlain = 0, kAux = 1, kSplit = 2 };
+
+template <bool A_MN, bool B_MN, int KIND>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_aux,
                  const PairParams p) {
+  constexpr bool AUX = KIND == kAux, SPLIT = KIND == kSplit;
   using L = Layout<AUX>;
   constexpr int STAGES = L::kStages;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -97,8 +102,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const int num_m = (p.M + 2 * BM - 1) / (2 * BM);
   const int num_n = (p.N + BN - 1) / BN;
   const int num_kb = (p.K + BK - 1) / BK;
-  const int full_tiles = num_m * num_n - p.tail_tiles;
-  const int num_items = full_tiles + p.tail_tiles * p.splits;
+  const int full_tiles = num_m * num_n - (SPLIT ? p.tail_tiles : 0);
+  const int num_items = full_tiles + (SPLIT ? p.tail_tiles * p.splits : 0);
   constexpr int GM = 4;  // 256-row tiles per raster group: neighbours share B panels in L2
 
   auto tile_coords = [&](int t, int& m0, int& n0) {
@@ -117,7 +122,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     kb0 = 0;
     kb1 = num_kb;
     split = -1;
-    if (w >= full_tiles) {
+    if (SPLIT && w >= full_tiles) {
       const int u = w - full_tiles;
       split = u / p.tail_tiles;
       t = full_tiles + u - split * p.tail_tiles;
@@ -283,7 +288,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
       };
       const float4* parts = nullptr;         // the tile's parts in K order, where it was split
-      if (!AUX && split >= 0) {
+      if (SPLIT && split >= 0) {
         constexpr int kPart4 = BM * BN / 4;  // float4s of a CTA's half of a part
         const int tail = t - full_tiles;
         float4* all = reinterpret_cast<float4*>(p.part) + static_cast<size_t>(tail) * p.splits * 2 * kPart4 + rank * kPart4 + r;
@@ -328,7 +333,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           for (int hh = 0; hh < halves; ++hh) {
             float v[32];
             const int col0 = ucol0 + hh * 32;
-            if (!AUX && parts) {
+            if (SPLIT && parts) {
               const float4* at = parts + (u * cols_per_unit + hh * 32) / 4 * BM;
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] = 0.f;
@@ -407,7 +412,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
       }
       aux_units += units_live;
-      if (AUX || split < 0) release_accumulator();
+      if (!SPLIT || split < 0) release_accumulator();
     }
     if (leader) tma_wait_all<0>();
   }
@@ -459,21 +464,24 @@ int g_sms = 0;
 struct Split {
   int tail_tiles, splits;
 };
-// How the last wave is cut.  A part costs its share of the K blocks, and 4 K blocks (of about 0.3 us) for each part that
-// is written and read back; a split has to save 8 K blocks.  So it is the long sums with a nearly empty last wave that
-// are split, above all weight gradients, whose K is the number of tokens: 16384 tokens, 7680 x 2560 (300 tiles on 74 pairs)
-// 490 -> 446 us; 8192 tokens, 4096 x 4096 (256 tiles) 208 -> 193 us, 4096 x 11008 (688 tiles) 700 -> 644 us.
+// How the last wave is cut.  Splitting saves the K blocks that a part leaves to others; against that stand the parts
+// written to memory and read back by one CTA in the end, and an epilogue that no longer overlaps anything: about 20 K blocks
+// and 12 more for each part, measured over 76 - 688 tiles, tails of 2 - 70 tiles, 8 - 256 K blocks and 2 - 8 parts.  Parts
+// that need a wave of their own never paid.  So it is the long sums with a nearly empty last wave that are split, above
+// all weight gradients, whose K is the number of tokens: of 256 K blocks 76 tiles (tail 2) 171 -> 134 us, 300 tiles (tail 4)
+// 491 -> 445; of 128 K blocks 76 tiles 90 -> 79 us, 256 tiles (tail 34) 208 -> 204.  Of 64 K blocks no tail gained (86 tiles,
+// tail 12: 47 -> 50 us), nor did a tail of 38 tiles of 128 (90 -> 96 us in three parts).
 Split choose_split(int M, int N, int K, int flags, int max_ctas) {
   Split none = {0, 1};
   const int pairs = max_ctas / 2, num_kb = (K + BK - 1) / BK;
   const long tiles = static_cast<long>((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
   if (pairs < 1 || tiles < pairs || (flags & (EPI_DGELU | EPI_RESIDUAL))) return none;
   const int tail = static_cast<int>(tiles % pairs);
-  int best = num_kb - 8, splits = 1;
-  for (int s = 2; s <= 8 && tail > 0 && num_kb / s >= 8; ++s) {
-    const int cost = (s * tail + pairs - 1) / pairs * ((num_kb + s - 1) / s) + 4 * (s + 1);
-    if (cost <= best) {
-      best = cost - 1;
+  int best = 12, splits = 1;
+  for (int s = 2; s <= 8 && tail > 0 && s * tail <= pairs && num_kb / s >= 8; ++s) {
+    const int gain = num_kb - (num_kb + s - 1) / s - 20 - 12 * s - tail * s / 10;
+    if (gain > best) {
+      best = gain;
       splits = s;
     }
   }
@@ -490,12 +498,12 @@ int clamp_ctas(int max_ctas) {
 }
 size_t arrived_bytes(const Split& s) { return (static_cast<size_t>(s.tail_tiles) * 2 * 4 + 255) / 256 * 256; }
 
-template <bool A_MN, bool B_MN, bool AUX>
+template <bool A_MN, bool B_MN, int KIND>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx,
            const PairParams& p, int max_ctas, cudaStream_t stream) {
-  constexpr int smem = Layout<AUX>::kTotal + 1024;
+  constexpr int smem = Layout<KIND == kAux>::kTotal + 1024;
   static bool configured = false;
-  auto kern = gemm_pair_kernel<A_MN, B_MN, AUX>;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, KIND>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
     configured = true;
@@ -520,13 +528,13 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tx, p) == cudaSuccess ? 0 : -4;
 }
 
-template <bool AUX>
+template <int KIND>
 int dispatch(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
              const CUtensorMap& tx, const PairParams& p, int max_ctas, cudaStream_t stream) {
-  if (!a_mn && !b_mn) return launch<false, false, AUX>(ta, tb, tc, tx, p, max_ctas, stream);
-  if (!a_mn && b_mn) return launch<false, true, AUX>(ta, tb, tc, tx, p, max_ctas, stream);
-  if (a_mn && !b_mn) return launch<true, false, AUX>(ta, tb, tc, tx, p, max_ctas, stream);
-  return launch<true, true, AUX>(ta, tb, tc, tx, p, max_ctas, stream);
+  if (!a_mn && !b_mn) return launch<false, false, KIND>(ta, tb, tc, tx, p, max_ctas, stream);
+  if (!a_mn && b_mn) return launch<false, true, KIND>(ta, tb, tc, tx, p, max_ctas, stream);
+  if (a_mn && !b_mn) return launch<true, false, KIND>(ta, tb, tc, tx, p, max_ctas, stream);
+  return launch<true, true, KIND>(ta, tb, tc, tx, p, max_ctas, stream);
 }
 
 }  // namespace
@@ -603,8 +611,9 @@ MB_API int mb_gemm_pair_split_bf16(const void* A, const void* B, void* C, int M,
   p.arrived = reinterpret_cast<int*>(workspace);
   p.part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + arrived_bytes(split));
   if (split.tail_tiles && cudaMemsetAsync(workspace, 0, arrived_bytes(split), stream) != cudaSuccess) return -4;
-  if (has_aux) return dispatch<true>(a_mn_major != 0, b_mn_major != 0, ta, tb, tc, tx, p, max_ctas, stream);
-  return dispatch<false>(a_mn_major != 0, b_mn_major != 0, ta, tb, tc, tx, p, max_ctas, stream);
+  if (has_aux) return dispatch<kAux>(a_mn_major != 0, b_mn_major != 0, ta, tb, tc, tx, p, max_ctas, stream);
+  if (split.tail_tiles) return dispatch<kSplit>(a_mn_major != 0, b_mn_major != 0, ta, tb, tc, tx, p, max_ctas, stream);
+  return dispatch<kPlain>(a_mn_major != 0, b_mn_major != 0, ta, tb, tc, tx, p, max_ctas, stream);
 }
 
 MB_API int mb_gemm_pair_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,

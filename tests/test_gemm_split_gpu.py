@@ -1,7 +1,8 @@
 """The CTA-pair GEMM with the tiles of its last wave cut along K, against 64 bits.
 
 Bounds: a bf16 result is rounded once (2^-9 of each value at most, 2^-8 allows for GELU's approximation beside it); an fp32
-result carries the rounding of a sum of K terms, about sqrt(K) * 2^-24 of the norm, for which 2e-5 leaves a factor of four."""
+result carries the error of the tensor core's fp32 sums, which grows with the number of terms: 1.86e-5 of the norm for an
+unsplit sum of 16384, the longest here, and less in parts.  2e-5 allows that."""
 import pytest
 import torch
 
@@ -12,8 +13,9 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-# M, N, K, a_mn, b_mn: two parts, five parts with a ragged K, ragged M and N (the second CTA of a pair past the bottom)
+# M, N, K, a_mn, b_mn: two parts, three with a ragged K, four; ragged M and N (the second CTA of a pair past the bottom)
 @pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(2560, 2560, 16384, True, True), (5632, 1024, 7000, True, True),
+                                             (4864, 1024, 16384, True, False),
                                              (2440, 2600, 8200, True, True), (2304, 2560, 8192, False, False),
                                              (2440, 2600, 8200, False, True)])
 @pytest.mark.parametrize("form", ["bf16", "accumulate", "bias_gelu_pre"])
