@@ -498,6 +498,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
 }
 
+#include "attn_fwd_one_tile_tcgen05.cuh"
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -560,8 +562,10 @@ MB_API int mb_attn_fwd(const void* q, const void* k, const void* v, void* o, flo
   if (units > 0x3fffffff) return -1;
   CUtensorMap tq, tk, tv;
   if (!make_map(&tq, q, batch, sq, nh, d, q_bs, q_ts, q_hs, BM)) return -2;
-  if (!make_map(&tk, k, batch, sk, nh_kv, d, k_bs, k_ts, k_hs, BN)) return -2;
-  if (!make_map(&tv, v, batch, sk, nh_kv, d, v_bs, v_ts, v_hs, BN)) return -2;
+  const bool small = one_tile::is_faster(sq, sk, static_cast<long>(nh) * batch, d) && nh <= 65535 && batch <= 65535;
+  const int bn = small ? one_tile::BN : BN;
+  if (!make_map(&tk, k, batch, sk, nh_kv, d, k_bs, k_ts, k_hs, bn)) return -2;
+  if (!make_map(&tv, v, batch, sk, nh_kv, d, v_bs, v_ts, v_hs, bn)) return -2;
   AttnParams p;
   p.o = reinterpret_cast<__nv_bfloat16*>(o);
   p.lse = lse;
@@ -574,6 +578,18 @@ MB_API int mb_attn_fwd(const void* q, const void* k, const void* v, void* o, flo
   p.seqlens_q = seqlens_q;
   p.seqlens_k = seqlens_k;
   p.status = mb_status_device_ptr();
+  if (small) {
+    static bool cfg = false;
+    if (!cfg) {
+      if (cudaFuncSetAttribute(one_tile::attn_fwd_one_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               one_tile::Smem::kTotal) != cudaSuccess)
+        return -3;
+      cfg = true;
+    }
+    one_tile::attn_fwd_one_tile_kernel<<<dim3((sq + BM - 1) / BM, nh, batch), one_tile::kThreads,
+                                         one_tile::Smem::kTotal, stream>>>(tq, tk, tv, p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  }
   static bool cfg = false;
   if (!cfg) {
     if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)

@@ -52,6 +52,18 @@ SHAPES = [  # b, sq, sk, heads, kv heads, d, causal
     (1, 384, 384, 3, 3, 112, False),
     (3, 640, 640, 40, 10, 80, True),       # more work items than CTAs, dQ beside dV and dK in tensor memory
     (2, 1024, 1024, 24, 4, 128, True),     # the same, dQ over dP
+    # both sides of the sizes at which the forward kernel of one tile per CTA takes over
+    (2, 64, 64, 3, 3, 64, True),
+    (2, 65, 64, 3, 3, 64, False),
+    (2, 32, 64, 4, 2, 128, True),
+    (2, 33, 64, 4, 2, 128, True),
+    (149, 32, 1024, 1, 1, 48, True),       # more heads than SMs: fewer queries than keys
+    (37, 64, 320, 4, 2, 64, False),
+    (37, 64, 100, 4, 4, 32, True),         # queries and keys of less than a tile, three key blocks of 64
+    (10, 128, 150, 15, 5, 32, True),
+    (75, 64, 64, 2, 2, 128, False),
+    (1, 192, 192, 4, 4, 64, True),         # two tiles, each on a CTA of its own
+    (1, 300, 64, 4, 4, 64, True),          # queries that see no key
 ]
 
 
@@ -75,13 +87,18 @@ def test_block_kernels_at_tile_edges(b, sq, sk, nh, nkv, d, causal):
         _close(got, want)
 
 
+# s, heads, kv heads, lengths: own heads; groups summed after the kernel, and inside it; short sequences
+@pytest.mark.parametrize("s,nh,nkv,lens", [(400, 6, 6, [400, 1, 128, 257]), (400, 6, 2, [400, 1, 128, 257]),
+                                           (640, 24, 8, [640, 129, 1, 500, 640, 64, 333, 256]),
+                                           (60, 6, 3, [60, 1, 33]), (32, 160, 160, [7, 32])])
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("d", [64, 128])
-def test_block_kernels_on_padded_batches(d, causal):
+def test_block_kernels_on_padded_batches(s, nh, nkv, lens, d, causal):
     torch.manual_seed(d)
-    b, s, nh = 4, 400, 6
-    q, k, v, g = (torch.randn(b, s, nh, d, device=DEV, dtype=torch.bfloat16) for _ in range(4))
-    lens = torch.tensor([400, 1, 128, 257], device=DEV, dtype=torch.int32)
+    b = len(lens)
+    q, g = (torch.randn(b, s, nh, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(b, s, nkv, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    lens = torch.tensor(lens, device=DEV, dtype=torch.int32)
     scale = 1 / math.sqrt(d)
     leaves = [t.double().requires_grad_(True) for t in (q, k, v)]
     o_ref, _ = _exact(*leaves, scale, causal, lens, lens)
@@ -108,4 +125,56 @@ def test_gradients_into_a_packed_projection(nh, nkv, s):
     o_ref.backward(g.double())
     _close(o, o_ref)
     for got, want in zip(qkv.grad.split([nh, nkv, nkv], 2), leaf.grad.split([nh, nkv, nkv], 2)):
+        _close(got, want)
+
+
+def _rotate(x, cos, sin, rot):
+    """The rotation in 64 bits: channels in halves, ``x`` ``[b, s, heads, d]``."""
+    c, sn = cos.double()[:, None], sin.double()[:, None]
+    x1, x2 = x[..., :rot // 2], x[..., rot // 2:rot]
+    return torch.cat([x1 * c - x2 * sn, x1 * sn + x2 * c, x[..., rot:]], -1)
+
+
+@pytest.mark.parametrize("nh,nkv,d,rot", [(4, 4, 64, 64), (6, 2, 80, 32), (8, 2, 128, 128)])
+@pytest.mark.parametrize("lens", [None, [300, 17, 129]])
+def test_projection_with_rotary_and_lengths(nh, nkv, d, rot, lens):
+    torch.manual_seed(d)
+    b, s = 3, 300
+    x = torch.randn(b, s, nh + 2 * nkv, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    g = torch.randn(b, s, nh, d, device=DEV, dtype=torch.bfloat16)
+    lens = None if lens is None else torch.tensor(lens, device=DEV, dtype=torch.int32)
+    cos, sin = F.rope_tables(s, rot, 10000.0, DEV)
+    scale = 1 / math.sqrt(d)
+    o = F.attention_projected(x.clone(), nkv, scale, True, (cos, sin, rot), lens)
+    o.backward(g)
+    native.check_status()
+    leaf = x.detach().double().requires_grad_(True)
+    q, k, v = leaf.split([nh, nkv, nkv], 2)
+    o_ref, _ = _exact(_rotate(q, cos, sin, rot), _rotate(k, cos, sin, rot), v, scale, True, lens, lens)
+    o_ref.backward(g.double())
+    # q and k are rounded to bf16 once more, behind the rotation, and so is their gradient: a third and a fourth rounding of
+    # 2^-9 each, independent of the two above
+    for got, want in zip((o, *x.grad.split([nh, nkv, nkv], 2)), (o_ref, *leaf.grad.split([nh, nkv, nkv], 2))):
+        diff = got.double() - want
+        assert torch.isfinite(got).all() and diff.norm() <= 2 ** -7.5 * want.norm()
+        assert diff.abs().max() <= 2 ** -6 * want.abs().max()
+
+
+@pytest.mark.parametrize("nh,nkv,d", [(4, 4, 64), (6, 2, 128)])
+@pytest.mark.parametrize("sq,sk", [(40, 300), (300, 40)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_packed_keys_and_values(nh, nkv, d, sq, sk, padded):
+    torch.manual_seed(sq)
+    b, scale = 2, 0.1
+    q = torch.randn(b, sq, nh, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    kv = torch.randn(b, sk, 2, nkv, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    g = torch.randn(b, sq, nh, d, device=DEV, dtype=torch.bfloat16)
+    lens_q, lens_k = (torch.tensor([n, n // 3], device=DEV, dtype=torch.int32) if padded else None for n in (sq, sk))
+    o = F.attention_kvpacked(q, kv, scale, False, lens_q, lens_k)
+    o.backward(g)
+    native.check_status()
+    q_ref, kv_ref = (t.detach().double().requires_grad_(True) for t in (q, kv))
+    o_ref, _ = _exact(q_ref, kv_ref[:, :, 0], kv_ref[:, :, 1], scale, False, lens_q, lens_k)
+    o_ref.backward(g.double())
+    for got, want in ((o, o_ref), (q.grad, q_ref.grad), (kv.grad, kv_ref.grad)):
         _close(got, want)
