@@ -560,7 +560,7 @@ int g_bwd_last_variant = 0;
 MB_API int* mb_status_device_ptr();
 
 // Chooses the main backward kernel for later calls: 0 = the kernel that finishes one 64-row query block
-// before it starts the next (default), 1 = the pipelined kernel on 128 x 128 blocks.
+// before it starts the next (default), 1 = the pipelined kernel on 128 x 128 blocks, but for the smallest problems.
 MB_API void mb_attn_bwd_set_variant(int v) { g_bwd_variant = (v == 1) ? 1 : 0; }
 // Variant the last call of mb_attn_bwd launched.
 MB_API int mb_attn_bwd_last_variant() { return g_bwd_last_variant; }
@@ -581,7 +581,10 @@ MB_API int mb_attn_bwd(const void* dout, const void* q, const void* k, const voi
                        long dk_bs, long dk_ts, long dk_hs, long dv_bs, long dv_ts, long dv_hs, float scale,
                        int causal, const int* seqlens_q, const int* seqlens_k, cudaStream_t stream) {
   if (d % 16 || d > 128 || d < 16) return -1;
-  const bool pipelined = g_bwd_variant == 1;
+  // A block or two per head and no more heads than SMs: the chain through one CTA is all there is, and it is shorter in the
+  // one-block kernel (8 heads of 64, 16 positions: 12.3 us with its three kernels against 13.5).
+  const bool tiny = sq <= 32 && sk <= 64 && nh == nh_kv && static_cast<long>(nh) * batch <= 128;
+  const bool pipelined = g_bwd_variant == 1 && !tiny;
   if (nh_kv < 1 || nh % nh_kv || unit_heads < 1 || (nh / nh_kv) % unit_heads || (!pipelined && nh != nh_kv)) return -1;
   if ((q_bs | q_ts | q_hs | k_bs | k_ts | k_hs | v_bs | v_ts | v_hs | dq_bs | dq_ts | dq_hs | dk_bs | dk_ts |
        dk_hs | dv_bs | dv_ts | dv_hs) & 7)

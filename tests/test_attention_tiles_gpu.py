@@ -44,6 +44,11 @@ def _close(got, want):
 
 SHAPES = [  # b, sq, sk, heads, kv heads, d, causal
     (1, 1, 1, 1, 1, 16, True),             # one row
+    (2, 32, 64, 64, 64, 64, False),        # the largest problem of the one-block backward kernel, and past it on each side
+    (2, 33, 64, 8, 8, 64, False),
+    (2, 32, 65, 8, 8, 128, True),
+    (3, 20, 20, 43, 43, 80, True),
+    (2, 20, 20, 8, 4, 96, True),
     (2, 127, 127, 2, 2, 64, True),         # one short of a tile
     (1, 129, 129, 2, 1, 80, True),         # one row in the second tile
     (1, 257, 257, 4, 2, 96, True),         # one row in a second pair of tiles
