@@ -1,8 +1,7 @@
-"""Model check of the barrier protocol of the attention forward kernel
-(``attn_fwd_kernel`` in mist_b200/csrc/attn_fwd_tcgen05.cu), for the default layout (one producer
-thread requests K and V) and the layout with a producer warp of its own for V.
+"""Model check of the barrier protocol of the attention forward kernel for short sequences
+(``attn_fwd_one_tile_kernel`` in mist_b200/csrc/attn_fwd_one_tile_tcgen05.cuh).
 
-Roles: producer(s), MMA issuer, softmax threads, the in-order tensor-core queue.  Per key block j
+Roles: producer, MMA issuer, softmax threads, the in-order tensor-core queue.  Per key block j
 (stage st = j % 2, score buffer b = j & 1):
 
     k_full[st], v_full[st]   producer -> MMA        the tile is in shared memory
@@ -14,8 +13,7 @@ Roles: producer(s), MMA issuer, softmax threads, the in-order tensor-core queue.
     pv_done                  MMA commit -> softmax  the PV product of block j is complete
 
 The simulation replays waits, arrivals and parities with random latencies and checks liveness and
-that no buffer is overwritten while in use.  It also shows what the second producer is for: with one
-producer the request for K of block j+1 waits behind V's stage of block j.
+that no buffer is overwritten while in use.
 """
 import os
 import sys
@@ -29,7 +27,7 @@ from protocol_sim import MBar, Resource, Sim, Task, TensorQueue  # noqa: E402
 STAGES = 2
 
 
-def simulate(n_blocks, seed, split, n_soft=3, slow=None, drop=(), tma=(0.5, 3.0)):
+def simulate(n_blocks, seed, n_soft=3, slow=None, drop=()):
     sim = Sim(seed)
     slow = slow or {}
 
@@ -55,31 +53,21 @@ def simulate(n_blocks, seed, split, n_soft=3, slow=None, drop=(), tma=(0.5, 3.0)
 
     def load(res, bar, j):
         res.write_begin(j)
-    
+
         def land():
             res.write_end(j)
             bar.arrive()
-        sim.at(lat("tma", *tma), land)
+        sim.at(lat("tma", 0.5, 3.0), land)
 
     def producer_kv():
         if n_blocks == 0:
             return
-        sim.at(lat("tma", *tma), q_full.arrive)
+        sim.at(lat("tma", 0.5, 3.0), q_full.arrive)
         for j in range(n_blocks):
             st = j % STAGES
             if j >= STAGES and "k_empty" not in drop:
                 yield ("wait", k_empty[st], ((j // STAGES) - 1) & 1)
             load(K[st], k_full[st], j)
-            if split:
-                continue
-            if j >= STAGES and "kv_empty" not in drop:
-                yield ("wait", kv_empty[st], ((j // STAGES) - 1) & 1)
-            load(V[st], v_full[st], j)
-            yield ("sleep", 0.01)
-
-    def producer_v():
-        for j in range(n_blocks):
-            st = j % STAGES
             if j >= STAGES and "kv_empty" not in drop:
                 yield ("wait", kv_empty[st], ((j // STAGES) - 1) & 1)
             load(V[st], v_full[st], j)
@@ -155,35 +143,30 @@ def simulate(n_blocks, seed, split, n_soft=3, slow=None, drop=(), tma=(0.5, 3.0)
                 O.read_end()
 
     tasks = [Task(sim, producer_kv(), "producer"), Task(sim, mma(), "mma")]
-    if split:
-        tasks.append(Task(sim, producer_v(), "producer_v"))
     tasks += [Task(sim, softmax(i), f"softmax{i}") for i in range(n_soft)]
     sim.run()
     stuck = [t.name for t in tasks if not t.done]
-    assert not stuck, f"n_blocks={n_blocks} seed={seed} split={split}: stuck roles {stuck}"
+    assert not stuck, f"n_blocks={n_blocks} seed={seed}: stuck roles {stuck}"
     if n_blocks > 0:
         assert p_full.completed == n_blocks and pv_done.completed == n_blocks
     return sim.t
 
 
-@pytest.mark.parametrize("split", [False, True])
 @pytest.mark.parametrize("n_blocks", [0, 1, 2, 3, 4, 7, 16])
-def test_forward_protocol_random_latencies(n_blocks, split):
+def test_forward_protocol_random_latencies(n_blocks):
     for seed in range(50):
-        simulate(n_blocks, seed, split)
+        simulate(n_blocks, seed)
 
 
-@pytest.mark.parametrize("split", [False, True])
 @pytest.mark.parametrize("role", ["tma", "mma", "soft"])
-def test_forward_protocol_with_one_slow_role(role, split):
+def test_forward_protocol_with_one_slow_role(role):
     for seed in range(20):
-        simulate(9, seed, split, slow={role: 20.0})
-        simulate(9, 500 + seed, split, slow={role: 0.05})
+        simulate(9, seed, slow={role: 20.0})
+        simulate(9, 500 + seed, slow={role: 0.05})
 
 
-@pytest.mark.parametrize("split", [False, True])
 @pytest.mark.parametrize("wait", ["k_empty", "kv_empty", "pv_done"])
-def test_forward_model_reports_a_hazard_when_a_wait_is_left_out(wait, split):
+def test_forward_model_reports_a_hazard_when_a_wait_is_left_out(wait):
     """Mutation check of the model.  (``s_empty`` is not in the list: the MMA warp issues S of block
     j+2 only after it has seen ``p_full`` of block j, which already implies that S of block j has been
     read, so that wait is redundant in the kernel and the model rightly reports nothing without it.)"""
@@ -191,17 +174,7 @@ def test_forward_model_reports_a_hazard_when_a_wait_is_left_out(wait, split):
     for seed in range(40):
         for slow in ({}, {"soft": 8.0}, {"mma": 8.0}, {"tma": 0.05}, {"tma": 8.0}):
             try:
-                simulate(9, seed, split, slow=slow, drop=(wait,))
+                simulate(9, seed, slow=slow, drop=(wait,))
             except AssertionError:
                 failures += 1
     assert failures > 0
-
-
-def test_second_producer_shortens_the_block_time_when_loads_take_longer_than_a_block():
-    """Load latency 2.0 against about 1.2 of softmax time per block: with one producer the request for K
-    of block j+1 goes out only once V's stage of block j is free, about one block before its S product,
-    and the pipeline waits for the load; with two producers it goes out a block earlier."""
-    n = 30
-    single = sum(simulate(n, s, False, n_soft=1, tma=(1.8, 2.2)) for s in range(10)) / 10
-    double = sum(simulate(n, s, True, n_soft=1, tma=(1.8, 2.2)) for s in range(10)) / 10
-    assert double < 0.95 * single
