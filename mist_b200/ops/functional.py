@@ -48,6 +48,7 @@ class Settings:
     """Process-wide kernel selection switches."""
     gemm_backend = "tcgen05"      # "tcgen05" (ours) | "cublas" (library, A/B baseline)
     attn_backend = "tcgen05"      # "tcgen05" (ours) | "sdpa" (library, A/B baseline)
+    attn_block_n = 64             # no effect, like attn_fwd's block_n: the kernels choose their key blocks by the sizes
     # Backward kernel on 128 x 128 blocks that overlaps the next block's S / dP products with the current block's
     # softmax; MIST_B200_ATTN_BWD_PIPELINED=0 selects the one that finishes a 64-row query block before the next.
     attn_bwd_pipelined = os.environ.get("MIST_B200_ATTN_BWD_PIPELINED", "1") != "0"
@@ -810,7 +811,7 @@ def _select_variant(setter: str, want: int):
 def attn_fwd(q, k, v, scale, causal, block_n=None, seqlens_q=None, seqlens_k=None):
     """Forward only: returns (o [b,sq,nh,d], lse [b,nh,sq] fp32).  ``seqlens_q`` / ``seqlens_k``: int32
     device tensors ``[b]`` with the number of real tokens of each sample of a right-padded batch.
-    ``block_n`` has no effect (the kernel has one block size); it is accepted for callers that pass it."""
+    ``block_n`` has no effect (the kernels choose by the sizes); it is accepted for callers that pass it."""
     if not use_native(q):
         return _ref_attention(q, k, v, scale, causal, seqlens_q, seqlens_k)
     b, sq, nh, d = q.shape

@@ -73,3 +73,9 @@ def test_qkvpacked_takes_strided_input():
     wide = torch.randn(2, 7, 3, 4, 24)
     ref = F.attention(wide[:, :, 0, :, :16], wide[:, :, 1, :, :16], wide[:, :, 2, :, :16])
     torch.testing.assert_close(F.attention_qkvpacked(wide[..., :16]), ref, rtol=1e-6, atol=1e-6)
+
+
+def test_block_size_settings_are_accepted():
+    q, k, v = (torch.randn(1, 5, 2, 16) for _ in range(3))
+    want, _ = F.attn_fwd(q, k, v, 0.25, True)
+    assert torch.equal(F.attn_fwd(q, k, v, 0.25, True, block_n=F.Settings.attn_block_n)[0], want)
