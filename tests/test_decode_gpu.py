@@ -155,3 +155,53 @@ def test_native_decode_step_matches_the_modules(model, extra, b, monkeypatch):
     assert _rel(got, want) < 2e-2
     for a, r in zip(cache, cache_ref):
         assert _rel(a, r) < 2e-2
+
+
+# batches of every token-tile size, the largest that the step takes, and a residual stream that comes in
+@pytest.mark.parametrize("model", ["gpt2/1.3b", "llama/1.3b"])
+@pytest.mark.parametrize("b,with_residual", [(3, True), (20, False), (65, True), (128, False)])
+def test_native_decode_step_takes_every_parameter(model, b, with_residual, monkeypatch):
+    """Biases on every linear and no two norms alike: each entry of the block's table has to arrive where it belongs."""
+    from mist_b200.config import load_config
+    from mist_b200.inference import kv_cache
+    from mist_b200.models.provider import base_model_provider
+    from mist_b200.models.transformer import ParallelTransformer
+    from mist_b200.ops import decode
+    cfg, _ = load_config("config", ["experiment=gpt2-1.3b", f"model={model}", "model.num_hidden_layers=2",
+                                    "model.hidden_size=512", "model.intermediate_size=1408",
+                                    "model.num_attention_heads=8", "model.vocab_size=1024", "model.qkv_proj_bias=true",
+                                    "model.out_proj_bias=true", "model.mlp_fc1_bias=true", "model.mlp_fc2_bias=true",
+                                    "training.max_sequence_length=64", "strategy.layer_partitions=[2]"],
+                         check_world_size=False)
+    torch.manual_seed(b)
+    net = base_model_provider(cfg.model, device=torch.device(DEV), dtype=torch.bfloat16).eval()
+    stack = next(m for m in net.modules() if type(m) is ParallelTransformer)
+    filled = 0
+    with torch.no_grad():
+        for name, p in stack.named_parameters():
+            if p.dim() == 1:
+                p.normal_(std=0.5).add_(1.0 if "norm" in name and name.endswith("weight") else 0.0)
+                filled += 1
+    assert filled >= 2 * (8 if model.startswith("gpt2") else 6)      # four biases and two norms a block
+    x, res = (torch.randn(3, b, 1, 512, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+
+    def steps():
+        with torch.no_grad(), kv_cache(net, b, 8) as ip:
+            out = []
+            for t in range(3):
+                out.append(stack(x[t], res[t] if with_residual else None).float())
+                ip.seqlen_offset += 1
+            return torch.stack(out), [ip.key_value_memory[i][:, :3].float() for i in range(2)]
+
+    calls = []
+    native_step = decode.stack_step
+    monkeypatch.setattr(decode, "stack_step", lambda *a: calls.append(native_step(*a)) or calls[-1])
+    got, cache = steps()
+    assert len(calls) == 3 and all(c is not None for c in calls)
+    monkeypatch.setattr(decode, "stack_step", lambda *a: None)
+    want, cache_ref = steps()
+    # Two blocks of about ten roundings of at most 2^-9 each, at different places on the two sides: a 2-norm below
+    # 2^-9 / sqrt(3) * sqrt(2 * 20), 0.7 %; a parameter in the wrong place changes half of the result and more.
+    assert _rel(got, want) < 2 ** -6
+    for a, r in zip(cache, cache_ref):
+        assert _rel(a, r) < 2 ** -6
