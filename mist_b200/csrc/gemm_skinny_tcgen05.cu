@@ -339,22 +339,25 @@ bool configure() {
 // a cluster share a GPC).  A constant, so that sums are cut the same way on every GPU.
 constexpr int kClusterSms[kMaxSplit + 1] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
 
-// CTAs that share a tile's K range: as many as leave each at least four K blocks (one ring) and the whole grid resident
+// CTAs that share a tile's K range: as many as leave each at least two K blocks and the whole grid resident
 // (three CTAs per SM with 16 columns, one with 128, whose stages are larger): a second wave costs more than shorter sums
 // give.  7680 x 2560 at 32 tokens (60 tiles): 4 CTAs a tile 11.7 us, 8 CTAs 19.4; 12288 x 4096 (96 tiles, at most 90
 // clusters of three): 2 CTAs a tile 22.4 us, 3 CTAs 29.0; 22016 x 4096 at one token (172 tiles): 2 CTAs a tile 31.2 us,
-// one 33.8.
+// one 33.8.  Against at least four K blocks each, in a chain of launches of 1 - 128 tokens: 1024 x 1024 5.0 -> 4.6 us at one
+// token and 8.4 -> 7.2 at 128, 512 x 512 4.6 -> 4.1 and 9.9 -> 7.8; the worst of 128 sizes 3072 x 1024 at 64 tokens, 7.1 -> 7.3.
+// Sums of fewer than eight K blocks stay whole: 128 x 256 took 3.3 us in one part, 4.1 in two.
 template <int NT>
 int choose_split(int tiles, int num_kb) {
   constexpr int per_sm = NT == 16 ? 3 : NT <= 64 ? 2 : 1;
-  int split = num_kb / 4 < kMaxSplit ? num_kb / 4 : kMaxSplit;
+  if (num_kb < 8) return 1;
+  int split = num_kb / 2 < kMaxSplit ? num_kb / 2 : kMaxSplit;
   while (split > 1 && kClusterSms[split] / split * per_sm < tiles) --split;
   return split < 1 ? 1 : split;
 }
 
 // Whether this kernel beats the tiled ones, which put the tokens on the 128-row side of the product; both sides measured
 // for N from 64 to 50304 and K from 64 to 50304.  Up to 32 tokens it does at every size (0.14 - 0.96 of their time).
-// Above, its epilogue needs enough K blocks to hide behind: at 64 tokens 512 x 512 took 7.5 us against 6.7 and
+// Above, its epilogue needs enough K blocks to hide behind: at 64 tokens 512 x 512 took 7.5 us in two parts against 6.7 and
 // 50304 x 1024 28.9 against 28.1, but 1024 x 1024 7.0 against 8.9.  Above 64 its stages leave one CTA per SM, and it has
 // to split K to win: 128 tokens, 4096 x 4096 16 us against 24, but 12288 x 4096 31 against 26.
 bool pays(int M, int num_kb, int split) {
